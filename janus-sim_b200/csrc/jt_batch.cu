@@ -191,8 +191,9 @@ struct Plan {
     std::vector<int> ids;                 // boxes of this pass
     std::vector<jt_seg_dev> pre, post;    // segments before / after the reorder
     std::vector<jt_box_dev> bx;
-    std::vector<int64_t> pprefix, iprefix, tprefix, gprefix, ptprefix, kprefix, cprefix, zprefix;
+    std::vector<int64_t> pprefix, iprefix, tprefix, gprefix, ptprefix, kprefix, zprefix;
     int64_t npart = 0, ninternal = 0, nsorttiles = 0, ngroups = 0, npmtiles = 0, nmodes = 0, ncells = 0;
+    int64_t ncols = 0;                    // columns of the near-field cell lists
     int64_t nztiles = 0;                  // CTAs of the fused z-transform kernel
     int zsizes = 0;                       // its grid sizes in the pass: bit 0 512^3, bit 1 256^3
     bool cells = false;                   // the near-field cell walk runs (jt_b_cells)
@@ -205,7 +206,7 @@ struct Plan {
     const jt_seg_dev* d_post = nullptr;
     const jt_box_dev* d_bx = nullptr;
     const int64_t *d_pp = nullptr, *d_ip = nullptr, *d_tp = nullptr, *d_gp = nullptr, *d_ptp = nullptr,
-                  *d_kp = nullptr, *d_cp = nullptr, *d_zp = nullptr;
+                  *d_kp = nullptr, *d_zp = nullptr;
 };
 
 float elapsed(cudaEvent_t a, cudaEvent_t b)
@@ -237,8 +238,9 @@ struct jt_batch {
     Pool<unsigned> cslot;
     Pool<float4> cpos;
     Pool<float4> pmacc;                 // PM accelerations of the pass, per interlaced grid
-    Pool<int2> cid;
-    Pool<unsigned char> tflag;
+    Pool<int2> cid, cmap;
+    Pool<unsigned char> tflag, cdense;
+    Pool<unsigned long long> creach;
     Pool<float4> com, bmin, bmax, quad0;
     Pool<float2> quad1;
     Pool<uint32_t> m30, vals, vals_alt, keys_alt, hist, status, tickets;
@@ -500,6 +502,33 @@ size_t put(std::vector<unsigned char>& buf, const std::vector<T>& v)
     return off;
 }
 
+// Columns per axis of a box's near-field cell list: side s such that 32
+// particles at the mean density fill a cube of side s (a batch of the cell
+// walk is then compact), at least cut / 1.9 (two columns on either side cover
+// the reach) and at most 256 per axis.
+int cell_columns(double L, double rcut, int64_t n)
+{
+    const double s = std::cbrt(32.0 / (double)n) * L;
+    const double q = std::min(L / s, 1.9 * L / rcut);
+    return q >= 256.0 ? 256 : (q < 1.0 ? 1 : (int)q);
+}
+
+// the cell list of a box with nb columns per axis
+void box_cells(jt_box_dev& d, int64_t n, int nb, const jt_config& c, double rcut)
+{
+    const double L = c.box_L;
+    d.nb = nb;
+    d.nbx = 8 * nb;
+    d.cell_inv = (float)(nb / L);
+    d.cellx_inv = (float)(d.nbx / L);
+    // the farthest column with a gap below the cut (1e-4 margin)
+    d.colm = (int)(rcut * 1.0001 * nb / L + 1.0e-4) + 1;
+    // JT_CELL_KMAX per 27 r_cut^3, in particles per bin
+    const double bin = L / nb * (L / nb) * (L / d.nbx);
+    d.cell_dmax = (float)(JT_CELL_KMAX / (27.0 * c.r_cut * c.r_cut * c.r_cut) * bin);
+    d.reach_max = (float)(JT_CELL_REACH / c.theta * (double)n);   // theta 0: no multipoles, never
+}
+
 // Size the scratch pools for the listed boxes, lay out their segments and
 // boxes, and upload every table in one copy.
 int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* steps, Plan& P)
@@ -558,7 +587,7 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
 
     int64_t o_node = 0, o_part = 0, o_tile = 0;
     P.pprefix.push_back(0); P.iprefix.push_back(0); P.tprefix.push_back(0); P.gprefix.push_back(0);
-    P.ptprefix.push_back(0); P.kprefix.push_back(0); P.cprefix.push_back(0); P.zprefix.push_back(0);
+    P.ptprefix.push_back(0); P.kprefix.push_back(0); P.zprefix.push_back(0);
     P.cells = cells_enabled();
     P.bx.resize(nb);
     for (int k = 0; k < nb; k++) {
@@ -616,26 +645,14 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
             P.screened = true;
         }
         d.seg[0] = d.seg[1] = -1;
-        // near-field cells of side L / nb >= r_cut (1e-4 margin against
-        // binning round-off); fewer than 3 per axis: tree walk only
-        d.nb = 0;
-        d.cbase = P.cprefix.back();
-        if (P.cells && rcut > 0.0) {
-            const double q = c.box_L / (rcut * 1.0001);
-            int nbc = q >= 256.0 ? 256 : (int)q;
-            if (nbc >= 3) d.nb = nbc;
-            if (d.nb && b->cell_nb >= 3 && b->cell_nb < d.nb) d.nb = b->cell_nb;   // timed (tune_cells)
-        }
-        // a widened cut scales every neighbourhood's count by (cut / r_cut)^3,
-        // and cells wider than the default by (default nb / nb)^3
-        {
-            const double w = rcut / c.r_cut;
-            const double q = d.nb ? c.box_L / (rcut * 1.0001) : 0.0;
-            const double v = d.nb ? std::min(256.0, std::floor(q)) / d.nb : 1.0;
-            d.cell_kmax = (int)std::min(1.0e6, JT_CELL_KMAX * std::max(1.0, w * w * w) * v * v * v);
-        }
-        d.cell_inv = d.nb ? (float)(d.nb / c.box_L) : 0.0f;
-        P.cprefix.push_back(P.cprefix.back() + (int64_t)d.nb * d.nb * d.nb);
+        // near-field cells where at least three cuts fit along the box; else
+        // tree walk only
+        d.cbase = P.ncells;
+        d.colbase = P.ncols;
+        if (P.cells && rcut > 0.0 && c.box_L >= 3.0 * 1.0001 * rcut)
+            box_cells(d, b->n[0] + b->n[1], b->cell_nb > 0 ? b->cell_nb : cell_columns(c.box_L, rcut, b->n[0] + b->n[1]), c, rcut);
+        P.ncells += (int64_t)d.nb * d.nb * d.nbx;
+        P.ncols += (int64_t)d.nb * d.nb;
         for (int s = 0; s < 2; s++) {
             const int64_t n = b->n[s];
             if (n == 0) continue;
@@ -691,7 +708,6 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
     P.npmtiles = P.ptprefix.back();
     P.nmodes = P.kprefix.back();
     P.nztiles = P.zprefix.back();
-    P.ncells = P.cprefix.back();
     if (P.cells) {
         JT_TRY(B->ccount.ensure((size_t)std::max<int64_t>(P.ncells, 1), &grew));
         JT_TRY(B->cstart.ensure((size_t)P.ncells + 1, &grew));
@@ -701,6 +717,9 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
         JT_TRY(B->cpos.ensure((size_t)std::max<int64_t>(P.npart, 1), &grew));
         JT_TRY(B->cid.ensure((size_t)std::max<int64_t>(P.npart, 1), &grew));
         JT_TRY(B->tflag.ensure((size_t)std::max<int64_t>(P.npart, 1), &grew));
+        JT_TRY(B->cdense.ensure((size_t)P.ncells / 8 + 1, &grew));
+        JT_TRY(B->creach.ensure((size_t)nb, &grew));
+        JT_TRY(B->cmap.ensure((size_t)(P.npart / 32 + P.ncols + 1), &grew));
         JT_TRY(B->csegflag.ensure((size_t)std::max<int>(nseg, 1), &grew));
     }
     if (!P.screened) JT_TRY(B->pmacc.ensure((size_t)B->ngrid * std::max<int64_t>(P.npart, 1), &grew));
@@ -710,7 +729,7 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
     size_t o_pre = put(buf, P.pre), o_post = put(buf, P.post), o_bx = put(buf, P.bx);
     size_t o_pp = put(buf, P.pprefix), o_ip = put(buf, P.iprefix), o_tp = put(buf, P.tprefix);
     size_t o_gp = put(buf, P.gprefix), o_ptp = put(buf, P.ptprefix), o_kp = put(buf, P.kprefix);
-    size_t o_cp = put(buf, P.cprefix), o_zp = put(buf, P.zprefix);
+    size_t o_zp = put(buf, P.zprefix);
     JT_TRY(B->desc.ensure(buf.size(), &grew));
     // the previous upload may still read the staging buffer
     JT_CU(cudaEventSynchronize(B->desc_done));
@@ -734,28 +753,27 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
     P.d_gp = (const int64_t*)(d + o_gp);
     P.d_ptp = (const int64_t*)(d + o_ptp);
     P.d_kp = (const int64_t*)(d + o_kp);
-    P.d_cp = (const int64_t*)(d + o_cp);
     P.d_zp = (const int64_t*)(d + o_zp);
     P.table_bytes = buf.size();
     return JT_OK;
 }
 
-// The cell walk's cost depends on how a cell's targets fill batches of 32
-// (a lattice whose points per cell are a whole number per axis fills them
-// evenly), which no model of the mean count predicts: the first force-only
-// pass of a box of kCellTuneMin particles or more, alone in its pass, times
-// the cell walk at every nb from the default (side >= cut) down to 0.8 of it
-// (the faster of two runs each) and keeps the fastest for the box (nb with
-// targets flagged for the tree walk are not taken: they would time less
-// work).  2x224^3 at cut 6 r_s: 68 -> 56 cells per axis (4 lattice points,
-// 128 particles), cell walk 5 % faster.  JT_CELL_TUNE=0 in the environment
-// (read once) keeps the default.
+// The cell walk's cost depends on how the columns cut the particle
+// distribution (a lattice whose points fall into the columns evenly gives
+// compact full batches), which no model of the mean count predicts: the first
+// force-only pass of a box of kCellTuneMin particles or more, alone in its
+// pass, times the cell walk at several column counts from the default down to
+// 0.7 of it (the faster of two runs each) and keeps the fastest for the box (a
+// count with targets flagged for the tree walk is not taken: it would time
+// less work).  JT_CELL_TUNE=0 in the environment (read once) keeps the default.
 constexpr int64_t kCellTuneMin = (int64_t)1 << 22;
 
 std::mutex g_cell_tune_mu;
 std::string g_cell_tune_text;   // one entry per timed box (jt_cell_tuning_text)
 
-int tune_cells(jt_batch* B, Plan& P, int nseg, int parts, const float4* pmacc)
+// *done: the pass's cell walk has already run (a clustered box keeps the default,
+// which the first timing run left in place).
+int tune_cells(jt_batch* B, Plan& P, int nseg, int parts, const float4* pmacc, bool* done)
 {
     jt_box_state* bs = B->boxes[P.ids[0]];
     jt_box_dev& d = P.bx[0];
@@ -770,57 +788,57 @@ int tune_cells(jt_batch* B, Plan& P, int nseg, int parts, const float4* pmacc)
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(B->st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return JT_OK;
     cudaStream_t st = B->st;
-    const int nmax = d.nb, kmax0 = d.cell_kmax, nmin = std::max(3, (int)std::ceil(0.8 * nmax));
-    jt_cell_bufs cb = {B->ccount.p, B->cstart.p, B->cbsum.p, B->ccell.p, B->cslot.p,
-                       B->cpos.p, B->cid.p, B->tflag.p, B->csegflag.p};
-    cudaEvent_t e0, e1;
-    JT_CU(cudaEventCreate(&e0));
-    if (cudaEventCreate(&e1) != cudaSuccess) {
-        cudaEventDestroy(e0);
-        return JT_ECUDA;
-    }
+    const int nmax = d.nb, nmin = std::max(3, (int)std::ceil(0.7 * nmax)), dn = std::max(1, nmax / 24);
+    const double rcut = jt_short_cut(bs->cfg);
+    jt_cell_bufs cb = {B->ccount.p, B->cstart.p, B->cbsum.p, B->ccell.p, B->cslot.p, B->cpos.p, B->cid.p, B->tflag.p,
+                       B->cdense.p, B->creach.p, B->cmap.p, B->csegflag.p};
+    const cudaEvent_t e0 = B->ev[8], e1 = B->ev[9];   // the pass's own events around the cell walk
     auto set_nb = [&](int nb) -> int {
-        const double v = (double)nmax / nb;
-        d.nb = nb;
-        d.cell_inv = (float)(nb / (double)d.L);
-        d.cell_kmax = (int)std::min(1.0e6, kmax0 * v * v * v);
-        P.cprefix[1] = (int64_t)nb * nb * nb;
-        P.ncells = P.cprefix[1];
-        if (cudaMemcpyAsync((void*)P.d_bx, &d, sizeof(jt_box_dev), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-            cudaMemcpyAsync((void*)(P.d_cp + 1), &P.cprefix[1], sizeof(int64_t), cudaMemcpyHostToDevice, st) !=
-                cudaSuccess)
+        box_cells(d, bs->n[0] + bs->n[1], nb, bs->cfg, rcut);
+        P.ncols = (int64_t)nb * nb;
+        P.ncells = P.ncols * d.nbx;
+        if (cudaMemcpyAsync((void*)P.d_bx, &d, sizeof(jt_box_dev), cudaMemcpyHostToDevice, st) != cudaSuccess)
             return JT_ECUDA;
         return JT_OK;
     };
     int r = JT_OK, best = nmax;
+    bool crowded = false;
     float best_ms = 0.f;
-    for (int nb = nmax; nb >= nmin && r == JT_OK; nb--) {
+    for (int nb = nmax; nb >= nmin && r == JT_OK; nb -= dn) {
         r = set_nb(nb);
         // two runs, the faster one counts (candidates a few % apart)
         float ms = 0.f;
         int flag[2] = {0, 0};
+        unsigned long long reach = 0;
         for (int rep = 0; rep < 2 && r == JT_OK; rep++) {
-            r = jt_b_cells(P.d_post, P.d_bx, P.d_pp, nseg, P.npart, P.d_cp, 1, P.ncells, cb, B->order, B->ngrid,
-                           parts, 0.0f, nullptr, B->d_err, st, e0, e1, false, pmacc, false);
+            r = jt_b_cells(P.d_post, P.d_bx, P.d_pp, nseg, P.npart, 1, P.ncells, P.npart / 32 + P.ncols, cb, B->order,
+                           B->ngrid, parts, 0.0f, nullptr, B->d_err, st, e0, e1, false, pmacc, false);
             if (r == JT_OK && (cudaMemcpyAsync(flag, B->csegflag.p, sizeof(int) * (size_t)nseg,
                                                cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+                               cudaMemcpyAsync(&reach, B->creach.p, sizeof(reach), cudaMemcpyDeviceToHost, st) !=
+                                   cudaSuccess ||
                                cudaStreamSynchronize(st) != cudaSuccess))
                 r = JT_ECUDA;
             float m = 0.f;
             if (r == JT_OK && cudaEventElapsedTime(&m, e0, e1) != cudaSuccess) r = JT_ECUDA;
             if (r == JT_OK && (rep == 0 || m < ms)) ms = m;
+            // crowded or clustered at the default already (the mean number of
+            // particles in reach twice that of a uniform box): keep it
+            if (r == JT_OK && nb == nmax) {
+                const double w = 2 * d.colm + 1, n = (double)(bs->n[0] + bs->n[1]);
+                const double uniform = std::min(1.0, w * w * std::min(w, (double)nb) / ((double)nb * nb * nb));
+                crowded = flag[0] || flag[1] || (double)reach > 2.0 * n * n * uniform;
+                if (crowded) break;
+            }
         }
-        if (r != JT_OK) break;
+        if (r != JT_OK || crowded) break;
         if (nb == nmax) {
             best_ms = ms;
-            if (flag[0] || flag[1]) break;   // crowded at the default already: keep it
         } else if (!flag[0] && !flag[1] && ms < best_ms) {
             best = nb;
             best_ms = ms;
         }
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     if (r != JT_OK) return r;
     bs->cell_nb = best;
     {
@@ -829,7 +847,8 @@ int tune_cells(jt_batch* B, Plan& P, int nseg, int parts, const float4* pmacc)
             g_cell_tune_text += "cells " + std::to_string(bs->n[0] + bs->n[1]) + " particles: " +
                                 std::to_string(nmax) + " -> " + std::to_string(best) + " per axis; ";
     }
-    return set_nb(best);
+    *done = crowded && !B->counters;
+    return *done ? JT_OK : set_nb(best);
 }
 
 // One force pass over the plan's boxes; afterwards every box's state sits in
@@ -906,13 +925,15 @@ int force_pass(jt_batch* B, Plan& P, int parts, float kick_frac)
         cudaEventRecord(B->ev[8], st);
         cudaEventRecord(B->ev[9], st);
     } else {
+        bool done = false;
         if (kick_frac == 0.0f && nbox == 1 && P.ncells > 0 && (parts & JT_PART_SHORT))
-            JT_TRY(tune_cells(B, P, nseg, parts, pmacc));
-        jt_cell_bufs cb = {B->ccount.p, B->cstart.p, B->cbsum.p, B->ccell.p, B->cslot.p,
-                           B->cpos.p, B->cid.p, B->tflag.p, B->csegflag.p};
-        JT_TRY(jt_b_cells(P.d_post, P.d_bx, P.d_pp, nseg, P.npart, P.d_cp, nbox, P.ncells, cb, B->order,
-                          B->ngrid, parts, kick_frac, B->d_stats, B->d_err, st, B->ev[8], B->ev[9],
-                          P.screened, pmacc, B->counters));
+            JT_TRY(tune_cells(B, P, nseg, parts, pmacc, &done));
+        jt_cell_bufs cb = {B->ccount.p, B->cstart.p, B->cbsum.p, B->ccell.p, B->cslot.p, B->cpos.p, B->cid.p,
+                           B->tflag.p, B->cdense.p, B->creach.p, B->cmap.p, B->csegflag.p};
+        if (!done)
+            JT_TRY(jt_b_cells(P.d_post, P.d_bx, P.d_pp, nseg, P.npart, nbox, P.ncells,
+                              P.ncells > 0 ? P.npart / 32 + P.ncols : 0, cb, B->order, B->ngrid, parts, kick_frac,
+                              B->d_stats, B->d_err, st, B->ev[8], B->ev[9], P.screened, pmacc, B->counters));
         tflag = B->tflag.p;
         jt_b_build_trees(P.d_post, P.d_bx, nseg, P.d_ip, P.ninternal, P.d_pp, P.npart, st, B->csegflag.p);
         B->tm.launches += P.npart > 0 ? (P.ncells > 0 ? 6 : 1) : 0;
@@ -1445,7 +1466,7 @@ void jt_batch_destroy(jt_batch* B)
     B->com.release(); B->bmin.release(); B->bmax.release(); B->quad0.release(); B->quad1.release();
     B->ccount.release(); B->cstart.release(); B->cbsum.release(); B->ccell.release(); B->cslot.release();
     B->csegflag.release();
-    B->cpos.release(); B->cid.release(); B->tflag.release(); B->pmacc.release();
+    B->cpos.release(); B->cid.release(); B->cmap.release(); B->cdense.release(); B->creach.release(); B->tflag.release(); B->pmacc.release();
     B->m30.release(); B->vals.release(); B->vals_alt.release(); B->keys_alt.release();
     B->hist.release(); B->status.release(); B->tickets.release(); B->desc.release();
     drop_graphs(B);
@@ -1764,9 +1785,10 @@ int jt_batch_estimate(const jt_config* cfg, size_t n_p, size_t n_m, size_t* pers
         size_t tree = 2 * n * (sizeof(int2) + sizeof(int) + 4 * sizeof(float4) + sizeof(float2)) +
                       n * (sizeof(int2) + sizeof(int));
         size_t sort = n * 4 * sizeof(uint32_t) + (n / 4096 + 2) * 4 * 256 * sizeof(uint32_t);
-        // near-field cell list (cpos, cid, ccell, cslot, tflag per particle)
-        // and the interpolated PM accelerations (one float4 per grid)
-        size_t cells = n * (sizeof(float4) + sizeof(int2) + 2 * sizeof(int) + 1) +
+        // near-field cell list (cpos, cid, ccell, cslot, tflag per particle;
+        // ccount, cstart and cmap about 3 bytes more) and the interpolated PM
+        // accelerations (one float4 per grid)
+        size_t cells = n * (sizeof(float4) + sizeof(int2) + 2 * sizeof(int) + 4) +
                        n * box_ngrid(*cfg) * sizeof(float4);
         *scratch = tree + sort + cells + grid_bytes(M, box_ngrid(*cfg));
     }
@@ -1799,7 +1821,7 @@ int jt_batch_trim(jt_batch* B)
     B->com.release(); B->bmin.release(); B->bmax.release(); B->quad0.release(); B->quad1.release();
     B->ccount.release(); B->cstart.release(); B->cbsum.release(); B->ccell.release(); B->cslot.release();
     B->csegflag.release();
-    B->cpos.release(); B->cid.release(); B->tflag.release(); B->pmacc.release();
+    B->cpos.release(); B->cid.release(); B->cmap.release(); B->cdense.release(); B->creach.release(); B->tflag.release(); B->pmacc.release();
     B->m30.release(); B->vals.release(); B->vals_alt.release(); B->keys_alt.release();
     B->hist.release(); B->status.release(); B->tickets.release();
     for (auto& kv : B->buckets) kv.second.release();

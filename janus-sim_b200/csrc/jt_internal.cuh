@@ -114,10 +114,15 @@ struct jt_box_dev {
     float2* force_s_k;
     float* force_s;
     const float2* ytab;   // the Yukawa kernel's log table (JT_LTAB_N entries)
-    int nb;               // cells per axis of the near-field cell list (0: tree walk only)
-    int cell_kmax;        // a cell whose 27-cell neighbourhood holds more goes to the tree walk
+    int nb;               // columns per axis (y, z) of the near-field cell list (0: tree walk only)
+    int nbx;              // bins of a column along x
+    int colm;             // columns in reach on either side of a batch's own (at most 2)
+    float cell_dmax;      // a block with more particles per bin in reach is dense (k_cell_dense)
+    float reach_max;      // the box's sum of particles in reach above which dense blocks go to the tree walk
     float cell_inv;       // nb / L
+    float cellx_inv;      // nbx / L
     int64_t cbase;        // this box's first cell in the pass's cell tables
+    int64_t colbase;      // this box's first column in the pass
 };
 
 __device__ __forceinline__ int jt_find(const int64_t* __restrict__ prefix, int count, int64_t i)
@@ -213,13 +218,21 @@ __device__ __forceinline__ float jt_wrap(float d, float L, float halfL)
     return d;
 }
 
-// Near-field cells whose 27-cell neighbourhood holds more candidates than
-// this (at the config's r_cut; scaled by (cut / r_cut)^3 for a widened cut)
-// send their targets to the tree walk: clustered data, where the dense
-// evaluation's cost grows with the square of the local count.
-#ifndef JT_CELL_KMAX
-#define JT_CELL_KMAX 2048
-#endif
+// In a strongly clustered box (mean particles in reach above JT_CELL_REACH /
+// theta) the tree walk takes the targets of the blocks that have more than
+// JT_CELL_KMAX particles per 27 r_cut^3 in reach; in other boxes the cell walk
+// takes every target.  The cell walk's time grows with the particles in
+// reach, the tree walk's only as about their square root (multipoles), and
+// mixing the two in one box of middling density costs more than either
+// alone (two kernels that each wait for a few long groups).  Measured, 2x64^3
+// particles in Plummer spheres (L 50, PM 128^3, near field of one force pass),
+// by mean particles in reach, cell walk alone against tree walk:
+//   10,200 (64 spheres):  3.3 ms against 5.8 / 5.1 / 4.3 at theta 0.3 / 0.5 / 0.7
+//   28,500 (16 spheres): 10.7 ms against 13.9 / 10.8 / 8.6
+//   45,500 (2x128^3, 64 spheres): 160 ms against 147 / 99 / 64
+//   83,800 (4 spheres):  39.5 ms against 27.8 / 17.2 / 12.3
+constexpr double JT_CELL_REACH = 13500.0;
+constexpr double JT_CELL_KMAX = 2048.0;
 
 // The short-range cut of an accurate-mode box: r_cut, or with cut_tail_ppm
 // = k > 0 the radius where S(r / 2 r_s) = k * 1e-6 when that is larger.
@@ -337,19 +350,24 @@ int jt_b_walk(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t
               const int64_t* d_pprefix = nullptr, const unsigned char* tflag = nullptr,
               bool screened = false, const int* segflag = nullptr, const float4* pmacc = nullptr,
               int64_t npart = 0);
-// Near-field cell list of a pass (cells of side >= r_cut, both species) and
-// the cell walk over it: particles of cells whose 27-cell neighbourhood holds
-// more than JT_CELL_KMAX candidates, and of boxes without a cell grid, are
-// flagged in tflag for the tree walk; the others get their acceleration (and
-// fused kick) here.  Scratch: ccount/cstart C + 1 ints, bsum, ccell/cslot,
-// cpos/cid one entry per particle.
+// Near-field cell list of a pass (columns along x cut into bins, both
+// species) and the cell walk over it in batches of 32 targets: the dense
+// blocks of strongly clustered boxes, and boxes without a cell grid, flag
+// their particles in tflag for the tree walk; the others get their
+// acceleration (and fused kick) here.  Scratch: ccount/cstart ncells + 1
+// ints, bsum, cmap nslots, dense ncells / 8, reach nbox, ccell/cslot, cpos/cid
+// one entry per particle.
+// nslots: npart / 32 + the columns of all boxes.
 struct jt_cell_bufs {
     int* ccount; int* cstart; int* bsum; int* ccell; unsigned* cslot;
     float4* cpos; int2* cid; unsigned char* tflag;
+    unsigned char* dense;         // per block of 8 bins: above the tree walk's density
+    unsigned long long* reach;    // per box: sum over its particles of the particles in reach
+    int2* cmap;                   // batch slot -> (box, column of the box), -1: none
     int* segflag;                 // per segment: some particle is flagged (its tree is built)
 };
 int jt_b_cells(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t* d_pprefix, int nseg,
-               int64_t npart, const int64_t* d_cprefix, int nbox, int64_t ncells, const jt_cell_bufs& cb,
+               int64_t npart, int nbox, int64_t ncells, int64_t nslots, const jt_cell_bufs& cb,
                int order, int ngrid, int parts, float kick_frac, unsigned long long* stats,
                unsigned* d_err, cudaStream_t st, cudaEvent_t ev_walk0, cudaEvent_t ev_walk1,
                bool screened = false, const float4* pmacc = nullptr, bool count_pairs = true);

@@ -30,9 +30,9 @@
 
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
-#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -114,9 +114,12 @@ __device__ float2 g_ltab[JT_LTAB_N];
 // Fill a log-indexed table of G(y) = S(sqrt y) / y^{3/2} (JT_LTAB_N entries):
 // octave e = -32..5, segment k = 0..511 covers [2^e (1 + k/512),
 // 2^e (1 + (k+1)/512)); entry (a, b) is the chord through G at its two
-// ends, so that G ~ a + b y inside it (relative error <= (h / y)^2 / 8 times
-// y^2 |G''| / G: about 2e-6 where G ~ y^{-3/2}, up to ~2e-5 at y ~ 5 where S
-// falls off as e^{-y}).  The last entry is the one every y >= 64 (and every
+// ends lowered by two thirds of its distance from G at the middle (the mean
+// of the parabola between them), so that G ~ a + b y inside it without bias
+// (relative error at most (h / y)^2 / 12 times y^2 |G''| / G: about 1.3e-6
+// where G ~ y^{-3/2}, up to ~1.3e-5 at y ~ 5 where S falls off as e^{-y}; the
+// chord itself lies above G everywhere, and sums of thousands of pairs carry
+// that on).  The last entry is the one every y >= 64 (and every
 // y < 2^-32, through the unsigned index wrap) is clamped to: S ~ 1e-28 there.
 template <class F>
 void fill_log_table(F S, float2* tab)
@@ -126,7 +129,8 @@ void fill_log_table(F S, float2* tab)
         for (int k = 0; k < 512; k++) {
             const double y0 = base + k * h, y1 = y0 + h;
             const double g0 = S(y0) / (y0 * std::sqrt(y0)), g1 = S(y1) / (y1 * std::sqrt(y1));
-            const double b = (g1 - g0) / h, a = g0 - b * y0;
+            const double ym = 0.5 * (y0 + y1), gm = S(ym) / (ym * std::sqrt(ym));
+            const double b = (g1 - g0) / h, a = g0 - b * y0 - (2.0 / 3.0) * (0.5 * (g0 + g1) - gm);
             tab[(e + 32) * 512 + k] = make_float2((float)a, (float)b);
         }
     }
@@ -728,7 +732,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_walk_acc(WalkArgs A)
     float ghx = 0.5f * (hix - lox), ghy = 0.5f * (hiy - loy), ghz = 0.5f * (hiz - loz);
 
     Acc3 pm = {0.f, 0.f, 0.f};
-    if ((P.parts & 1) && !A.pmacc) pm = pm_interp<ORDER, NG>(B, p);
+    if (SCR && (P.parts & 1)) pm = pm_interp<ORDER, NG>(B, p);   // no tile interpolation in a screened pass
 
     Acc3 near = {0.f, 0.f, 0.f}, far = {0.f, 0.f, 0.f}, comp = {0.f, 0.f, 0.f};
     unsigned pairs = 0, nodes = 0, cands = 0;   // per lane (warp totals < 2^32)
@@ -743,7 +747,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_walk_acc(WalkArgs A)
                                      far, comp, pairs, nodes, cands, wc);
 
     if (valid && mine) {
-        if ((P.parts & 1) && A.pmacc) pm = pm_from_tiles<NG>(A.pmacc, A.npart, A.pprefix[g] + i);
+        if (!SCR && (P.parts & 1)) pm = pm_from_tiles<NG>(A.pmacc, A.npart, A.pprefix[g] + i);
         float ax = sgn_s * pm.x + near.x + (far.x - comp.x);
         float ay = sgn_s * pm.y + near.y + (far.y - comp.y);
         float az = sgn_s * pm.z + near.z + (far.z - comp.z);
@@ -1109,23 +1113,17 @@ int stab_ready()
 
 namespace {
 
-// ---- walk autotuner --------------------------------------------------------
-// The default launch shape of the walk (80 registers, 6 blocks per SM,
-// 32-particle leaf buckets) is the best measured at 2x224^3; other densities,
-// clustering and box mixes can prefer another register budget or bucket.  For
-// the default PM scheme (PCS, interlaced) the first force-only pass of each
-// size class (device, log2 of the warp-group count) times every variant once
-// and keeps the fastest; JT_WALK_VARIANT=<k> pins variant k.  Passes that kick
-// (the walk then updates velocities) or run under stream capture use the
-// cached or the default variant.
+// ---- tree walk launch shapes -----------------------------------------------
+// Resident blocks per SM the registers are sized for, and the leaf bucket.
+// Boxes of up to 2^19 warp groups run best at 96 registers (5 blocks per SM),
+// larger ones at 80 (6 blocks).  (Timing the variants on a process's first
+// force pass of a size picked an arbitrary one wherever that pass sent no
+// particle to the tree walk.)  JT_WALK_VARIANT=<k> pins variant k.
 struct WalkVariant {
     int minb, bkt;
 };
 constexpr WalkVariant kVariants[] = {{6, 32}, {5, 32}, {6, 24}};
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
-
-std::mutex g_tune_mu;
-std::map<std::pair<int, int>, int> g_tuned;   // (device, log2 groups) -> variant
 
 // the variants of the default PM scheme (PCS, interlaced)
 void launch_variant(int v, unsigned g, const WalkArgs& A, cudaStream_t st)
@@ -1137,57 +1135,13 @@ void launch_variant(int v, unsigned g, const WalkArgs& A, cudaStream_t st)
     }
 }
 
-int pick_variant(unsigned g, int64_t ngroups, const WalkArgs& A, cudaStream_t st)
+int pick_variant(int64_t ngroups)
 {
     if (const char* e = std::getenv("JT_WALK_VARIANT")) {
         const int v = std::atoi(e);
         return v >= 0 && v < kNumVariants ? v : 0;
     }
-    int dev = 0;
-    cudaGetDevice(&dev);
-    int lg = 0;
-    while (((int64_t)1 << (lg + 1)) <= ngroups) lg++;
-    const std::pair<int, int> key(dev, lg);
-    {
-        std::lock_guard<std::mutex> lock(g_tune_mu);
-        auto it = g_tuned.find(key);
-        if (it != g_tuned.end()) return it->second;
-    }
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (A.kick_frac != 0.0f || cudaStreamIsCapturing(st, &cs) != cudaSuccess ||
-        cs != cudaStreamCaptureStatusNone)
-        return 0;
-    // time each variant on this pass (force only: every run writes the same
-    // accelerations); statistics are left to the real launch
-    WalkArgs T = A;
-    T.stats = nullptr;
-    cudaEvent_t e0, e1;
-    if (cudaEventCreate(&e0) != cudaSuccess) return 0;
-    if (cudaEventCreate(&e1) != cudaSuccess) {
-        cudaEventDestroy(e0);
-        return 0;
-    }
-    int best = 0;
-    float best_ms = 0.f;
-    for (int v = 0; v < kNumVariants; v++) {
-        cudaEventRecord(e0, st);
-        launch_variant(v, g, T, st);
-        cudaEventRecord(e1, st);
-        float ms = 0.f;
-        if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) {
-            best = 0;
-            break;
-        }
-        if (v == 0 || ms < best_ms) {
-            best = v;
-            best_ms = ms;
-        }
-    }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    std::lock_guard<std::mutex> lock(g_tune_mu);
-    g_tuned[key] = best;
-    return best;
+    return ngroups <= ((int64_t)1 << 19) ? 1 : 0;
 }
 
 }  // namespace
@@ -1196,14 +1150,6 @@ extern "C" int jt_walk_tuning(char* buf, size_t len)
 {
     if (!buf || len == 0) return JT_EINVAL;
     std::string out;
-    {
-        std::lock_guard<std::mutex> lock(g_tune_mu);
-        for (const auto& kv : g_tuned) {
-            const WalkVariant& w = kVariants[kv.second];
-            out += "dev" + std::to_string(kv.first.first) + " groups~2^" + std::to_string(kv.first.second) +
-                   ": minblocks " + std::to_string(w.minb) + " bucket " + std::to_string(w.bkt) + "; ";
-        }
-    }
     out += jt_cell_tuning_text();
     std::snprintf(buf, len, "%s", out.c_str());
     return JT_OK;
@@ -1212,25 +1158,32 @@ extern "C" int jt_walk_tuning(char* buf, size_t len)
 namespace {
 
 // ------------------------------------------------------------------ cell walk
-// The near field as a cell list: per box a grid of nb^3 cells of side
-// L / nb >= r_cut (1e-4 margin), holding both species; every pair inside
-// r_cut lies in a cell and its 26 neighbours (nb >= 3, so the 27 are
-// distinct and the shifted image is the one within r_cut).  One warp per
-// cell: its targets (both species, ~30 at the 2x224^3 density) test every
-// candidate of the 27 cells that lies within r_cut of their AABB, in dense
-// chunks of 32 where every lane evaluates every candidate with the pair
-// force selected by r^2 < r_cut^2 (no per-lane hit loop, no traversal).
+// The near field as a cell list: per box nb x nb columns along x (side s =
+// L / nb on y and z), each cut into nbx bins along x (nbx = 8 nb), holding
+// both species.  The list is ordered by column, then bin, so a column's
+// particles run along x and any 32 consecutive ones of a column (a batch) are
+// a compact group: s is chosen so that 32 particles at the box's mean density
+// fill a cube of side s (box_cells in jt_batch.cu).  One warp takes a batch,
+// one target per lane; only a column's last batch has idle lanes.  (Cells of
+// side >= r_cut with one warp per cell left 25-40 % of the lanes idle where a
+// cell's count is no multiple of 32, and tested 27 whole cells per batch,
+// three times the candidates that the box test keeps.)
+// The warp takes the columns that its targets' bounding box reaches, in each
+// the bins within the reach left along x (periodic images as further
+// ranges), tests their particles against the box and evaluates the kept ones
+// in dense chunks of 32 where every lane evaluates every candidate with the
+// pair force selected by r^2 < r_cut^2 (no per-lane hit loop, no traversal).
 // Pairs are exactly those of the tree walk when it accepts no multipole
-// (the uniform case); cells whose neighbourhood holds more than
-// JT_CELL_KMAX candidates (clustered data) flag their particles for the
-// tree walk, which keeps its multipoles there.
+// (the uniform case); a strongly clustered box flags the targets of its dense
+// blocks for the tree walk, which keeps its multipoles there (k_cell_dense).
+// A pass with few batches splits each among the four warps of a block
+// (jt_b_cells): every fourth column each, the sums added in shared memory.
 
 struct CellArgs {
     const jt_seg_dev* segs;
     const jt_box_dev* boxes;
     const int64_t* pprefix;
-    int nseg, nbox;
-    const int64_t* cprefix;       // cells per box (nbox + 1)
+    int nseg;
     jt_cell_bufs cb;
     int parts;
     float kick_frac;
@@ -1265,9 +1218,9 @@ __global__ void k_cell_key(CellArgs A, int64_t npart)
     }
     const float4 p = SG.pos[i - A.pprefix[g]];
     const int nb = B.nb;
-    const int cx = cell_of(p.x, B.halfL, B.cell_inv, nb), cy = cell_of(p.y, B.halfL, B.cell_inv, nb),
+    const int cx = cell_of(p.x, B.halfL, B.cellx_inv, B.nbx), cy = cell_of(p.y, B.halfL, B.cell_inv, nb),
               cz = cell_of(p.z, B.halfL, B.cell_inv, nb);
-    const int key = (int)(B.cbase + ((int64_t)cz * nb + cy) * nb + cx);
+    const int key = (int)(B.cbase + ((int64_t)cz * nb + cy) * B.nbx + cx);
     // one atomic per distinct cell of the warp (Morton-ordered particles
     // mostly share their lanes' cells); slots follow lane order in a group
     const unsigned peers = __match_any_sync(__activemask(), key);
@@ -1280,8 +1233,10 @@ __global__ void k_cell_key(CellArgs A, int64_t npart)
     A.cb.tflag[i] = 0;
 }
 
-// exclusive scan of n counts, 1024 per block: block-local scan and block sums
-constexpr int kScanB = 1024;
+// exclusive scan of n counts (a multiple of 8), 4096 per block of 1024
+// threads: block-local scan and block sums, then each block adds the sums
+// before its own
+constexpr int kScanT = 1024, kScanB = 4 * kScanT;
 __device__ __forceinline__ int block_excl_scan(int v, int* wsum, int& total)
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1309,42 +1264,97 @@ __device__ __forceinline__ int block_excl_scan(int v, int* wsum, int& total)
     return before + x - v;
 }
 
-__global__ void k_scan_local(const int* __restrict__ in, int* __restrict__ out, int64_t n, int* __restrict__ bsum)
+__global__ void __launch_bounds__(kScanT) k_scan_local(const int* __restrict__ in, int* __restrict__ out, int64_t n,
+                                                       int* __restrict__ bsum)
 {
     __shared__ int wsum[32];
-    const int64_t i = (int64_t)blockIdx.x * kScanB + threadIdx.x;
-    const int v = i < n ? in[i] : 0;
+    const int64_t i = (int64_t)blockIdx.x * kScanB + 4 * threadIdx.x;
+    const int4 v = i < n ? *reinterpret_cast<const int4*>(in + i) : make_int4(0, 0, 0, 0);
     int total;
-    const int e = block_excl_scan(v, wsum, total);
-    if (i < n) out[i] = e;
+    const int e = block_excl_scan(v.x + v.y + v.z + v.w, wsum, total);
+    if (i < n) *reinterpret_cast<int4*>(out + i) = make_int4(e, e + v.x, e + v.x + v.y, e + v.x + v.y + v.z);
     if (threadIdx.x == 0) bsum[blockIdx.x] = total;
 }
 
-// one block: exclusive scan of the block sums in place (chunks of 1024 with
-// a running carry); bsum[nblk] = grand total
-__global__ void k_scan_sums(int* __restrict__ bsum, int nblk)
+// every block sums the totals before its own (a few thousand at most at the
+// sizes a device holds: no scan of them by a single block between the two
+// passes); the last one writes the grand total to out[n]
+__global__ void __launch_bounds__(kScanT) k_scan_add(int* __restrict__ out, int64_t n, const int* __restrict__ bsum)
 {
     __shared__ int wsum[32];
-    int carry = 0;
-    for (int base = 0; base < nblk; base += kScanB) {
-        const int i = base + threadIdx.x;
-        const int v = i < nblk ? bsum[i] : 0;
-        int total;
-        const int e = block_excl_scan(v, wsum, total);
-        if (i < nblk) bsum[i] = carry + e;
-        carry += total;
+    int before = 0, total;
+    for (int j = threadIdx.x; j < (int)blockIdx.x; j += kScanT) before += bsum[j];
+    block_excl_scan(before, wsum, total);
+    const int64_t i = (int64_t)blockIdx.x * kScanB + 4 * threadIdx.x;
+    if (i < n) {
+        int4 v = *reinterpret_cast<int4*>(out + i);
+        v.x += total;
+        v.y += total;
+        v.z += total;
+        v.w += total;
+        *reinterpret_cast<int4*>(out + i) = v;
     }
-    if (threadIdx.x == 0) bsum[nblk] = carry;
+    if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) out[n] = total + bsum[blockIdx.x];
 }
 
-__global__ void k_scan_add(int* __restrict__ out, int64_t n, const int* __restrict__ bsum, int nblk)
+// How crowded each block of 8 bins (a cube of side s) is: the particles
+// within colm blocks of it on every axis, about what its targets have in
+// reach.  cb.dense marks blocks above the tree walk's density (cell_dmax per
+// bin), cb.reach sums particles times particles in reach over each box: the
+// cost of walking all of it directly, which decides whether the box uses the
+// tree walk for its dense blocks (jt_box_dev.reach_max).  Both follow from the
+// counts alone, not from the order that the atomics gave the list.
+// One warp per block (per consecutive blocks at large sizes: one atomic for
+// all of them), one lane per column in reach.
+__global__ void __launch_bounds__(256) k_cell_dense(const jt_box_dev* __restrict__ boxes, int nbox, int64_t nblocks,
+                                                    int per, jt_cell_bufs cb)
 {
-    const int64_t i = (int64_t)blockIdx.x * kScanB + threadIdx.x;
-    if (i < n) out[i] += bsum[blockIdx.x];
-    if (i == 0) out[n] = bsum[nblk];
+    const int lane = threadIdx.x & 31;
+    const int64_t q0 = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * per;
+    const int64_t q1 = q0 + per < nblocks ? q0 + per : nblocks;
+    if (q0 >= nblocks) return;   // whole warp
+    int b = 0, hi = nbox - 1;    // the last box that starts at or before the block's first bin
+    while (b < hi) {
+        const int mid = (b + hi + 1) >> 1;
+        if (boxes[mid].cbase <= 8 * q0) b = mid; else hi = mid - 1;
+    }
+    unsigned long long work = 0;
+    for (int64_t q = q0; q < q1; q++) {
+        if (b + 1 < nbox && boxes[b + 1].cbase <= 8 * q) {   // into the next box (an empty grid adds no block)
+            if (lane == 0 && work) atomicAdd(cb.reach + b, work);
+            work = 0;
+            while (b + 1 < nbox && boxes[b + 1].cbase <= 8 * q) b++;
+        }
+        const jt_box_dev& B = boxes[b];
+        const int nb = B.nb, m = B.colm, w = 2 * m + 1;
+        const int* __restrict__ cstart = cb.cstart + B.cbase;
+        const int64_t local = q - B.cbase / 8;
+        const int n = cstart[8 * local + 8] - cstart[8 * local];
+        bool dense = false;
+        if (n > 0) {
+            const int kx = (int)(local % nb), cy = (int)((local / nb) % nb), cz = (int)(local / ((int64_t)nb * nb));
+            const int span = min(w, nb);   // blocks along x
+            const int x0 = w > nb ? 0 : kx - m, x1 = x0 + span;
+            int tot = 0;
+            if (lane < w * w) {
+                const int dy = lane % w - m, dz = lane / w - m;
+                const int* __restrict__ c = cstart + ((int64_t)((cz + dz + nb) % nb) * nb + (cy + dy + nb) % nb) * B.nbx;
+                tot = c[8 * min(x1, nb)] - c[8 * max(x0, 0)];
+                if (x0 < 0) tot += c[8 * nb] - c[8 * (nb + x0)];
+                if (x1 > nb) tot += c[8 * (x1 - nb)] - c[0];
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+            dense = (float)tot > B.cell_dmax * (float)(8 * span * w * w);
+            work += (unsigned long long)n * (unsigned long long)tot;
+        }
+        if (lane == 0) cb.dense[q] = dense ? 1 : 0;
+    }
+    if (lane == 0 && work) atomicAdd(cb.reach + b, work);
 }
 
-// particles into cell order: (x, y, z, s m) and (segment, index)
+// particles into cell order: (x, y, z, s m) and (segment, index; ~index for the
+// tree walk's targets); the batches
 __global__ void k_cell_scatter(CellArgs A, int64_t npart)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1359,151 +1369,349 @@ __global__ void k_cell_scatter(CellArgs A, int64_t npart)
     const float sm = SG.species == 0 ? B.mass[0] : -B.mass[1];
     const int dst = A.cb.cstart[key] + (int)A.cb.cslot[i];
     A.cb.cpos[dst] = make_float4(p.x, p.y, p.z, sm);
-    A.cb.cid[dst] = make_int2(g, (int)idx);
+    // a clustered box: the tree walk takes the targets of dense blocks
+    const bool dense = (float)A.cb.reach[SG.box] > B.reach_max && A.cb.dense[key >> 3];
+    A.cb.cid[dst] = make_int2(g, dense ? ~(int)idx : (int)idx);
+    if (dense) {
+        A.cb.tflag[i] = 1;
+        // the tree walk of a flagged particle walks both species' trees
+        if (B.seg[0] >= 0) A.cb.segflag[B.seg[0]] = 1;
+        if (B.seg[1] >= 0) A.cb.segflag[B.seg[1]] = 1;
+    }
+    // the first particle of each batch of 32 enters the batch in cmap.  A
+    // column c (counted over the pass's boxes) that starts at particle t0
+    // owns the slots from t0 / 32 + c: the next column's first slot lies at
+    // least ceil(count / 32) further, so no prefix sum of batch counts is needed
+    const int col = (int)((key - B.cbase) / B.nbx);
+    const int t0 = A.cb.cstart[B.cbase + (int64_t)col * B.nbx];
+    if (((dst - t0) & 31) == 0) A.cb.cmap[(t0 >> 5) + B.colbase + col + ((dst - t0) >> 5)] = make_int2(SG.box, col);
 }
 
-// A cell with more targets than one batch takes them in a spatial order:
-// sub-cell Morton code (3 bits per axis) of each target, ranked in shared
-// memory, so that each batch of 32 covers a compact part of the cell and
-// streams only the candidates its box can reach.  Cells with more than
-// kCellSortMax targets keep the list's order.
-constexpr int kCellSortMax = 256;
+constexpr int kCellRanges = 75;   // 25 columns, each with up to 3 images along x
 
 struct CellWarpSmem {
-    float4 cand[64];
-    int2 nrange[27];              // (first, count) of each neighbour cell
-    float4 nshift[27];            // periodic shift of its particles
-    int key[kCellSortMax];        // sub-cell code << 8 | target's rank in the list
-    int order[kCellSortMax];      // batch position -> target offset in the cell
+    // staged candidates, one array per component: cell_chunk reads four
+    // candidates of a component with one 16-byte load, two packed pairs
+    __align__(16) float cx[64], cy[64], cz[64], cq[64];
+    float4 shift[kCellRanges];    // periodic shift of a range's particles
+    int2 range[kCellRanges];      // (first, count)
 };
 
-// dense evaluation of candidates [0, cnt) for this lane's target: every pair
-// computed, the force selected by r^2 < r_cut^2.  Per pair: y = (r^2 + eps^2)
-// c^2 indexes the log table by its float bits and G(y) = a + b y (no
-// reciprocal square root, no float-int conversion); the lane accumulates
-// q_j G(y) d, which the caller scales by s_i c^3.  The target itself (r = 0,
-// d = 0) adds nothing and is counted as a hit, which the caller removes.
+// groups of four candidates in flight: 4 against 2 is 0.5-1.5 % faster
+constexpr int kCellUnroll = 4;
+
+// Two floats in one 64-bit register pair, for the packed FP32 instructions
+// (one issue slot for two operations; each half rounds as the scalar one).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// A lane's target for cell_chunk: coordinates negated and doubled into packed
+// pairs, and its sums.
+struct CellTarget {
+    f32x2 nx, ny, nz, ye, c2;
+    float si, yc;
+    float ax, ay, az;
+};
+
+// Two candidates' forces into the lane's sums, one after the other: the sums
+// run in the list's order whatever the filter of the batch let through (what
+// it drops would add exactly 0), so that two targets at one point get the same
+// bits in different batches of a column.
+__device__ __forceinline__ void add_pair(CellTarget& T, f32x2 w, f32x2 dx, f32x2 dy, f32x2 dz)
+{
+    const float2 ww = unpack2(w), x = unpack2(dx), y = unpack2(dy), z = unpack2(dz);
+    T.ax = fmaf(ww.x, x.x, T.ax);
+    T.ay = fmaf(ww.x, y.x, T.ay);
+    T.az = fmaf(ww.x, z.x, T.az);
+    T.ax = fmaf(ww.y, x.y, T.ax);
+    T.ay = fmaf(ww.y, y.y, T.ay);
+    T.az = fmaf(ww.y, z.y, T.az);
+}
+
+// The table entry of y when the pair is inside the cut, as a predicated load
+// (a branch around the load would keep the compiler from overlapping the
+// loads of several candidates); outside it (a, b) keep what they held.
+__device__ __forceinline__ void ld_inside(float2& ab, const float2* __restrict__ tab, float y, float yc)
+{
+    const float2* at = tab + ((__float_as_uint(y) >> 14) - JT_LTAB_BASE);
+    asm("{\n\t.reg .pred p;\n\tsetp.lt.f32 p, %2, %3;\n\t@p ld.global.nc.v2.f32 {%0, %1}, [%4];\n\t}"
+        : "+f"(ab.x), "+f"(ab.y)
+        : "f"(y), "f"(yc), "l"(at));
+}
+
+// dense evaluation of the staged candidates [0, cnt), cnt a multiple of 4,
+// for this lane's target: every pair computed, the force selected by r^2 <
+// r_cut^2.  Per pair: y = (r^2 + eps^2) c^2 indexes the log table by its
+// float bits and G(y) = a + b y (no reciprocal square root, no float-int
+// conversion); the lane accumulates q_j G(y) d, which the caller scales by
+// s_i c^3.  The target itself (r = 0, d = 0) adds nothing and is counted as a
+// hit, which the caller removes.
 // SCR: opposite-species pairs read the box's Yukawa table yt.
 // CNT: count the lane's pairs inside the cut (the pair counters; one
 // instruction per candidate, off unless the caller asks for them).
-// Positions come scaled by c = 1 / (2 r_s), so that y = |d|^2 + ye directly
-// (ye = eps^2 c^2) and the pair is inside the cut for y < yc.  No clamp on
+// y = r^2 c^2 + ye (c = 1 / (2 r_s), ye = eps^2 c^2), and the pair is inside
+// the cut for y < yc.  The differences are of the positions as they are
+// (scaling them by c when they are staged saves half a slot per candidate,
+// but its rounding, of the size of a coordinate's ulp, sets the error of
+// close pairs: 1e-5 of the force inside a clump against 1.5e-6).  No clamp on
 // the table index: the caller bounds ye >= 2^-32 and yc < 64, so that every
 // y of a lane inside the cut indexes the table ([2^-32, 2^6)); lanes outside
 // it load nothing.
+// What bounds it: issue slots (76 % issuing with scalar arithmetic and 25 slots
+// per candidate, filter included), then the latency of the table loads and the
+// L1 wavefronts of their gathers (73 % of peak now, 66 % issuing, 21 slots).
+// The differences, y and the weights of two candidates take one packed FP32
+// instruction each; the packed unit runs at half the scalar rate, so the FMA
+// pipe's time is unchanged.  Together with the batches (above): 2x224^3
+// 12.8 -> 9.2 ms at a cut of 4.5 r_s and 21.5 -> 16.6 ms at 6 r_s, 2x96^3
+// 0.86 -> 0.62 ms, 2 x 16^3 0.126 -> 0.023 ms.
 template <bool SCR, bool CNT>
-__device__ __forceinline__ unsigned cell_chunk(const float4* __restrict__ cand, int cnt, const float4& p, float si,
-                                               float yc, float ye, Acc3& a, const float2* __restrict__ yt)
+__device__ __forceinline__ unsigned cell_chunk(const CellWarpSmem& S, int cnt, CellTarget& T,
+                                               const float2* __restrict__ yt)
 {
     unsigned hits = 0;
-#pragma unroll 4
-    for (int j = 0; j < cnt; j++) {
-        const float4 q = cand[j];
-        const float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
-        const float y = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, ye)));
-        const unsigned k = (__float_as_uint(y) >> 14) - JT_LTAB_BASE;
-        const float2* __restrict__ tb = (SCR && si * q.w < 0.0f) ? yt : g_ltab;
-        const bool in = y < yc;
-        // only lanes inside the cut read the table (a predicated load: the
-        // ~3/4 of dense candidates outside it issue no L1 request), and the
-        // others' weight is selected to zero (one select instead of zeroing
-        // the load's registers)
-        float2 ab;
-        if (in) ab = __ldg(&tb[k]);
-        const float w = in ? q.w * fmaf(ab.y, y, ab.x) : 0.0f;
-        if (CNT) hits += in ? 1u : 0u;
-        a.x = fmaf(w, dx, a.x);
-        a.y = fmaf(w, dy, a.y);
-        a.z = fmaf(w, dz, a.z);
+#pragma unroll kCellUnroll
+    for (int j = 0; j < cnt; j += 4) {
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(S.cx + j);
+        const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(S.cy + j);
+        const ulonglong2 z = *reinterpret_cast<const ulonglong2*>(S.cz + j);
+        const float4 q = *reinterpret_cast<const float4*>(S.cq + j);
+        const f32x2 dxa = add2(x.x, T.nx), dya = add2(y.x, T.ny), dza = add2(z.x, T.nz);
+        const f32x2 dxb = add2(x.y, T.nx), dyb = add2(y.y, T.ny), dzb = add2(z.y, T.nz);
+        const float2 ya = unpack2(fma2(fma2(dza, dza, fma2(dya, dya, mul2(dxa, dxa))), T.c2, T.ye));
+        const float2 yb = unpack2(fma2(fma2(dzb, dzb, fma2(dyb, dyb, mul2(dxb, dxb))), T.c2, T.ye));
+        // only lanes inside the cut read the table (the ~2/3 of dense
+        // candidates outside it issue no L1 request)
+        float2 t0 = make_float2(0.f, 0.f), t1 = t0, t2 = t0, t3 = t0;
+        ld_inside(t0, SCR && T.si * q.x < 0.0f ? yt : g_ltab, ya.x, T.yc);
+        ld_inside(t1, SCR && T.si * q.y < 0.0f ? yt : g_ltab, ya.y, T.yc);
+        ld_inside(t2, SCR && T.si * q.z < 0.0f ? yt : g_ltab, yb.x, T.yc);
+        ld_inside(t3, SCR && T.si * q.w < 0.0f ? yt : g_ltab, yb.y, T.yc);
+        if (CNT)
+            hits += (ya.x < T.yc ? 1u : 0u) + (ya.y < T.yc ? 1u : 0u) + (yb.x < T.yc ? 1u : 0u) +
+                    (yb.y < T.yc ? 1u : 0u);
+        const f32x2 wa = mul2(pack2(q.x, q.y), pack2(fmaf(t0.y, ya.x, t0.x), fmaf(t1.y, ya.y, t1.x)));
+        const f32x2 wb = mul2(pack2(q.z, q.w), pack2(fmaf(t2.y, yb.x, t2.x), fmaf(t3.y, yb.y, t3.x)));
+        add_pair(T, wa, dxa, dya, dza);
+        add_pair(T, wb, dxb, dyb, dzb);
     }
     return hits;
 }
 
-// One batch of a cell's targets: lane l takes target base + l.  Smaller
-// batches (16 or 8 targets, the warp's lanes split into 2 or 4 candidate
-// streams) test 19 % or 37 % fewer candidates, but each batch streams and
-// tests the 27 neighbour cells again: measured 5 % and 33 % slower at
-// 2x224^3.  (Two targets per lane for cells with more than 32, which streams
-// and tests their candidates once instead of twice, measured slower too: its
-// registers lowered the occupancy of the whole kernel.)
-// base: the batch's first position in the cell's target order; t0, t1: the
-// cell's range of the cell list; sorted: the order comes from S.order
-template <int ORDER, int NG, bool SCR, bool CNT>
-__device__ __forceinline__ void cell_batch(const CellArgs& A, const jt_box_dev& B, CellWarpSmem& S, int base,
-                                           int t0, int t1, bool sorted, int lane, unsigned& pairs,
-                                           unsigned& cands)
+// resident blocks the registers are sized for: 7 (72 registers) hides more of
+// the table loads' latency than 6 (80: 2x96^3 0.62 against 0.61 ms) and spills
+// less than 8 (64: 0.66 ms)
+constexpr int kCellMinBlocks = 7;
+// SPLIT: the warps that share a batch (1, or the block's kWarps)
+template <int ORDER, int NG, bool SCR, bool CNT, int SPLIT>
+__global__ void __launch_bounds__(kWarps * 32, kCellMinBlocks) k_walk_cell(CellArgs A, int64_t nslots)
 {
+    __shared__ CellWarpSmem smem_all[kWarps];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int part = SPLIT > 1 ? wib : 0;
+    CellWarpSmem& S = smem_all[wib];
+    const int64_t slot = SPLIT > 1 ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * kWarps + wib;
+    if (slot >= nslots) return;   // whole warp; with SPLIT the whole block (as the returns below)
+    const int2 where = A.cb.cmap[slot];
+    if (where.x < 0) return;      // no batch in this slot
+    const jt_box_dev& B = A.boxes[where.x];
+    const int nb = B.nb, nbx = B.nbx, col = where.y;
+    const int* __restrict__ cstart = A.cb.cstart + B.cbase;
+    const int tc = cstart[(int64_t)col * nbx], t1 = cstart[(int64_t)(col + 1) * nbx];
+    const int t0 = tc + 32 * (int)(slot - ((tc >> 5) + B.colbase + col));
+    // an index below 0 marks a target of the tree walk (k_cell_scatter); a lane
+    // without a target of its own evaluates the batch's first that has one
+    const unsigned live = __ballot_sync(0xffffffffu, t0 + lane < t1 && A.cb.cid[t0 + lane].y >= 0);
+    if (!live) return;   // with SPLIT the whole block
+    const int t = (live >> lane) & 1u ? t0 + lane : t0 + __ffs(live) - 1;
     const unsigned lt = (1u << lane) - 1u;
     // the table covers y in [2^-32, 2^6): a softening below 2^-16 (2 r_s)
     // is raised to it, and the cut is bounded by y < 64 (16 r_s without
-    // softening), where the split factor is below 1e-27: the table's last
-    // entry, zero, held every y past it
-    const float cc = B.c, c2 = cc * cc, ye = fmaxf(B.eps2 * c2, 2.3283064365386963e-10f);
-    const float yc = fminf(fmaf(B.rc2, c2, ye), 64.0f * 0.99999f);
-    const float slack = B.halfL * 9.5367431640625e-7f, rc2_keep = B.rc2 * 1.00001f;
-    const float2* __restrict__ yt = (SCR && B.ytab) ? B.ytab : g_ltab;
-    const int pos_in_cell = base + lane;
-    const bool valid = t0 + pos_in_cell < t1;
-    const int t = t0 + (valid ? (sorted ? S.order[pos_in_cell] : pos_in_cell) : (sorted ? S.order[base] : base));
-    const float4 p = A.cb.cpos[t];
-    const int2 id = A.cb.cid[t];
-    const float si = p.w > 0.f ? 1.0f : -1.0f;
-    const float lox = warp_min(p.x), loy = warp_min(p.y), loz = warp_min(p.z);
-    const float hix = warp_max(p.x), hiy = warp_max(p.y), hiz = warp_max(p.z);
-    const float gcx = 0.5f * (lox + hix), gcy = 0.5f * (loy + hiy), gcz = 0.5f * (loz + hiz);
-    const float ghx = 0.5f * (hix - lox) + slack, ghy = 0.5f * (hiy - loy) + slack,
-                ghz = 0.5f * (hiz - loz) + slack;
+    // softening), where the split factor is below 1e-27
+    const float cc = B.c, c2 = cc * cc;
+    float si;
     Acc3 near = {0.f, 0.f, 0.f};
-    if (A.parts & 2) {
-        const float4 ps = make_float4(p.x * cc, p.y * cc, p.z * cc, p.w);
-        unsigned hits = 0;
-        int nc = 0;
-        for (int nbr = 0; nbr < 27; nbr++) {
-            const int2 r = S.nrange[nbr];
-            const float4 sh = S.nshift[nbr];
-            for (int o = 0; o < r.y; o += 32) {
-                bool keep = false;
-                float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (o + lane < r.y) {
-                    c = A.cb.cpos[r.x + o + lane];
-                    c.x += sh.x;
-                    c.y += sh.y;
-                    c.z += sh.z;
-                    const float gx = gap1(c.x - gcx, ghx), gy = gap1(c.y - gcy, ghy), gz = gap1(c.z - gcz, ghz);
-                    keep = gx * gx + gy * gy + gz * gz <= rc2_keep;
+    unsigned hits = 0, cands = 0;
+    {
+        const float4 p = A.cb.cpos[t];
+        si = p.w > 0.f ? 1.0f : -1.0f;
+        // the targets' box, padded by 8 ulp of the largest coordinate
+        const float slack = B.halfL * 9.5367431640625e-7f, rc2_keep = B.rc2 * 1.00001f;
+        const float lox = warp_min(p.x), loy = warp_min(p.y), loz = warp_min(p.z);
+        const float hix = warp_max(p.x), hiy = warp_max(p.y), hiz = warp_max(p.z);
+        const float gcx = 0.5f * (lox + hix), gcy = 0.5f * (loy + hiy), gcz = 0.5f * (loz + hiz);
+        const float ghx = 0.5f * (hix - lox) + slack, ghy = 0.5f * (hiy - loy) + slack,
+                    ghz = 0.5f * (hiz - loz) + slack;
+        // the columns in reach, one per lane: offsets -m .. m on y and z
+        // (m <= 2), each with its gap to the box; the reach left along x
+        // gives its bins, for the column itself and its images along x
+        int nr = 0;
+        {
+            const int m = B.colm, w = 2 * m + 1;
+            const int dy = lane % w - m, dz = lane / w - m;
+            const float side = B.L / (float)nb;
+            int ny = col % nb + dy, nz = col / nb + dz;
+            const float gy = gap1((ny + 0.5f) * side - B.halfL - gcy, ghy + 0.5f * side),
+                        gz = gap1((nz + 0.5f) * side - B.halfL - gcz, ghz + 0.5f * side);
+            const float rem = rc2_keep - gy * gy - gz * gz;
+            const bool reach = lane < w * w && rem >= 0.0f;
+            // a split batch's warps share its columns by their offset, the
+            // same for every batch of the column
+            const bool own = SPLIT == 1 || (lane & (SPLIT - 1)) == part;
+            float sy = 0.f, sz = 0.f;
+            if (ny < 0) { ny += nb; sy = -B.L; } else if (ny >= nb) { ny -= nb; sy = B.L; }
+            if (nz < 0) { nz += nb; sz = -B.L; } else if (nz >= nb) { nz -= nb; sz = B.L; }
+            const float rx = sqrtf(fmaxf(rem, 0.0f)) + ghx;
+            const int64_t c0 = ((int64_t)nz * nb + ny) * nbx;
+#pragma unroll
+            for (int k = -1; k <= 1; k++) {
+                const float lo = gcx - rx - k * B.L, hi = gcx + rx - k * B.L;
+                int first = 0, cnt = 0;
+                if (reach && lo <= B.halfL && hi >= -B.halfL) {
+                    first = cstart[c0 + cell_of(lo, B.halfL, B.cellx_inv, nbx)];
+                    cnt = cstart[c0 + cell_of(hi, B.halfL, B.cellx_inv, nbx) + 1] - first;
                 }
+                const unsigned has = __ballot_sync(0xffffffffu, own && cnt > 0);
+                if (own && cnt > 0) {
+                    const int at = nr + __popc(has & lt);
+                    S.range[at] = make_int2(first, cnt);
+                    S.shift[at] = make_float4(k * B.L, sy, sz, 0.f);
+                }
+                nr += __popc(has);
+            }
+        }
+        __syncwarp();
+        if ((A.parts & 2) && nr > 0) {
+            const float ye = fmaxf(B.eps2 * c2, 2.3283064365386963e-10f);
+            const float2* __restrict__ yt = (SCR && B.ytab) ? B.ytab : g_ltab;
+            CellTarget T;
+            T.nx = pack2(-p.x, -p.x);
+            T.ny = pack2(-p.y, -p.y);
+            T.nz = pack2(-p.z, -p.z);
+            T.ye = pack2(ye, ye);
+            T.c2 = pack2(c2, c2);
+            T.si = si;
+            T.yc = fminf(fmaf(B.rc2, c2, ye), 64.0f * 0.99999f);
+            T.ax = T.ay = T.az = 0.0f;
+            // groups of 32 candidates over all ranges; the next group is
+            // loaded while this one is tested and evaluated
+            int nc = 0, r = 0, o = 0;
+            int2 rg = S.range[0];
+            float4 nxt = lane < rg.y ? A.cb.cpos[rg.x + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+            while (r < nr) {
+                float4 c = nxt;
+                const float4 sh = S.shift[r];
+                const bool live = o + lane < rg.y;
+                o += 32;
+                if (o >= rg.y) {
+                    o = 0;
+                    if (++r < nr) rg = S.range[r];
+                }
+                if (r < nr && o + lane < rg.y) nxt = A.cb.cpos[rg.x + o + lane];
+                c.x += sh.x;
+                c.y += sh.y;
+                c.z += sh.z;
+                const float gx = gap1(c.x - gcx, ghx), gy = gap1(c.y - gcy, ghy), gz = gap1(c.z - gcz, ghz);
+                const bool keep = live && gx * gx + gy * gy + gz * gz <= rc2_keep;
                 const unsigned km = __ballot_sync(0xffffffffu, keep);
-                if (keep) S.cand[nc + __popc(km & lt)] = make_float4(c.x * cc, c.y * cc, c.z * cc, c.w);
+                if (keep) {
+                    const int at = nc + __popc(km & lt);
+                    S.cx[at] = c.x;
+                    S.cy[at] = c.y;
+                    S.cz[at] = c.z;
+                    S.cq[at] = c.w;
+                }
                 nc += __popc(km);
                 __syncwarp();
                 if (nc >= 32) {
-                    hits += cell_chunk<SCR, CNT>(S.cand, 32, ps, si, yc, ye, near, yt);
+                    hits += cell_chunk<SCR, CNT>(S, 32, T, yt);
                     cands += 32;
+                    // the entries past the chunk (distinct from those it
+                    // held) move to the front
+                    const float4 t2 = make_float4(S.cx[32 + lane], S.cy[32 + lane], S.cz[32 + lane], S.cq[32 + lane]);
                     __syncwarp();
-                    const float4 t2 = S.cand[32 + lane];
-                    __syncwarp();
-                    if (lane < nc - 32) S.cand[lane] = t2;
                     nc -= 32;
+                    if (lane < nc) {
+                        S.cx[lane] = t2.x;
+                        S.cy[lane] = t2.y;
+                        S.cz[lane] = t2.z;
+                        S.cq[lane] = t2.w;
+                    }
                     __syncwarp();
                 }
             }
+            if (nc > 0) {
+                // pad to a multiple of 4 with points outside any cut (< L / 2)
+                if (lane < ((-nc) & 3)) {
+                    S.cx[nc + lane] = gcx + 4.0f * B.L;
+                    S.cy[nc + lane] = gcy;
+                    S.cz[nc + lane] = gcz;
+                    S.cq[nc + lane] = 0.0f;
+                }
+                __syncwarp();
+                hits += cell_chunk<SCR, CNT>(S, (nc + 3) & ~3, T, yt);
+                cands += nc;
+            }
+            const float sc = si * c2 * cc;
+            near = Acc3{T.ax * sc, T.ay * sc, T.az * sc};
         }
-        if (nc > 0) {
-            hits += cell_chunk<SCR, CNT>(S.cand, nc, ps, si, yc, ye, near, yt);
-            cands += nc;
-        }
-        __syncwarp();
-        // the target met itself once (r = 0 < r_cut); an empty slot counts nothing
-        if (CNT && valid) pairs += hits - 1u;
-        const float sc = si * c2;   // positions scaled by c: sum w (c d)
-        near.x *= sc;
-        near.y *= sc;
-        near.z *= sc;
     }
-    if (valid) {
+    if (SPLIT > 1) {
+        __shared__ float sum[SPLIT > 1 ? SPLIT - 1 : 1][3][32];
+        if (part > 0) {
+            sum[part - 1][0][lane] = near.x;
+            sum[part - 1][1][lane] = near.y;
+            sum[part - 1][2][lane] = near.z;
+        }
+        __syncthreads();
+        if (part == 0) {
+#pragma unroll
+            for (int k = 0; k < SPLIT - 1; k++) {
+                near.x += sum[k][0][lane];
+                near.y += sum[k][1][lane];
+                near.z += sum[k][2][lane];
+            }
+        }
+    }
+    // read again: not held in registers over the candidates
+    const int2 id = A.cb.cid[t];
+    const bool valid = t == t0 + lane;   // its own target
+    if (valid && part == 0) {
         Acc3 pm = {0.f, 0.f, 0.f};
+        const float4 p = A.cb.cpos[t];
+        // a pass with a screened box has no tile interpolation
         if (A.parts & 1)
-            pm = A.pmacc ? pm_from_tiles<NG>(A.pmacc, A.npart, A.pprefix[id.x] + id.y) : pm_interp<ORDER, NG>(B, p);
+            pm = SCR ? pm_interp<ORDER, NG>(B, p) : pm_from_tiles<NG>(A.pmacc, A.npart, A.pprefix[id.x] + id.y);
         const jt_seg_dev& SG = A.segs[id.x];
         float ax = si * pm.x + near.x, ay = si * pm.y + near.y, az = si * pm.z + near.z;
         if (SCR && B.force_s && (A.parts & 1)) {
@@ -1529,89 +1737,13 @@ __device__ __forceinline__ void cell_batch(const CellArgs& A, const jt_box_dev& 
             SG.vel[id.y] = v;
         }
     }
-}
-
-#ifndef JT_CELL_MINB
-#define JT_CELL_MINB 6
-#endif
-template <int ORDER, int NG, bool SCR, bool CNT>
-__global__ void __launch_bounds__(kWarps * 32, JT_CELL_MINB) k_walk_cell(CellArgs A, int64_t ncells)
-{
-    __shared__ CellWarpSmem smem_all[kWarps];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    CellWarpSmem& S = smem_all[wib];
-    const int64_t gc = (int64_t)blockIdx.x * kWarps + wib;
-    if (gc >= ncells) return;   // whole warp
-    const int t0 = A.cb.cstart[gc], t1 = A.cb.cstart[gc + 1];
-    if (t0 == t1) return;
-    const int k = jt_find(A.cprefix, A.nbox, gc);
-    const jt_box_dev& B = A.boxes[k];
-    const int nb = B.nb;
-    const int64_t local = gc - A.cprefix[k];
-    const int cx = (int)(local % nb), cy = (int)((local / nb) % nb), cz = (int)(local / ((int64_t)nb * nb));
-    // the 27 neighbour cells: lane l < 27 takes offset (l % 3 - 1, l / 3 % 3 - 1, l / 9 - 1)
-    int cnt = 0;
-    if (lane < 27) {
-        int nx = cx + lane % 3 - 1, ny = cy + (lane / 3) % 3 - 1, nz = cz + lane / 9 - 1;
-        float sx = 0.f, sy = 0.f, sz = 0.f;
-        if (nx < 0) { nx += nb; sx = -B.L; } else if (nx >= nb) { nx -= nb; sx = B.L; }
-        if (ny < 0) { ny += nb; sy = -B.L; } else if (ny >= nb) { ny -= nb; sy = B.L; }
-        if (nz < 0) { nz += nb; sz = -B.L; } else if (nz >= nb) { nz -= nb; sz = B.L; }
-        const int64_t key = B.cbase + ((int64_t)nz * nb + ny) * nb + nx;
-        const int first = A.cb.cstart[key];
-        cnt = A.cb.cstart[key + 1] - first;
-        S.nrange[lane] = make_int2(first, cnt);
-        S.nshift[lane] = make_float4(sx, sy, sz, 0.f);
-    }
-    int tot = cnt;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-    if (tot > B.cell_kmax) {   // clustered: the tree walk takes these targets
-        for (int t = t0 + lane; t < t1; t += 32) {
-            const int2 id = A.cb.cid[t];
-            A.cb.tflag[A.pprefix[id.x] + id.y] = 1;
-        }
-        // the tree walk of a flagged particle walks both species' trees
-        if (lane == 0 && B.seg[0] >= 0) A.cb.segflag[B.seg[0]] = 1;
-        if (lane == 0 && B.seg[1] >= 0) A.cb.segflag[B.seg[1]] = 1;
-        return;
-    }
-    __syncwarp();
-    // more than one batch: rank the targets by sub-cell code (3 bits per
-    // axis, Morton order) so that consecutive batches are compact
-    const int nt = t1 - t0;
-    const bool sorted = nt > 32 && nt <= kCellSortMax;
-    if (sorted) {
-        const float cs = B.L / (float)nb;
-        const float ox = (float)cx * cs - B.halfL, oy = (float)cy * cs - B.halfL, oz = (float)cz * cs - B.halfL;
-        const float sc = 8.0f / cs;
-        for (int i = lane; i < nt; i += 32) {
-            const float4 q = A.cb.cpos[t0 + i];
-            const int ux = min(max((int)((q.x - ox) * sc), 0), 7), uy = min(max((int)((q.y - oy) * sc), 0), 7),
-                      uz = min(max((int)((q.z - oz) * sc), 0), 7);
-            int code = 0;
-#pragma unroll
-            for (int b = 0; b < 3; b++)
-                code |= (((ux >> b) & 1) << (3 * b)) | (((uy >> b) & 1) << (3 * b + 1)) | (((uz >> b) & 1) << (3 * b + 2));
-            S.key[i] = (code << 8) | i;   // unique: ties by list order
-        }
-        __syncwarp();
-        for (int i = lane; i < nt; i += 32) {
-            const int ki = S.key[i];
-            int rank = 0;
-            for (int j = 0; j < nt; j++) rank += S.key[j] < ki ? 1 : 0;
-            S.order[rank] = i;
-        }
-        __syncwarp();
-    }
-    unsigned pairs = 0, cands = 0;
-    for (int base = 0; base < nt; base += 32)
-        cell_batch<ORDER, NG, SCR, CNT>(A, B, S, base, t0, t1, sorted, lane, pairs, cands);
     if (A.stats) {
+        // a target met itself once (r = 0 < r_cut); an empty slot counts nothing
+        int pairs = CNT && valid ? (int)hits - (part == 0 && (A.parts & 2) ? 1 : 0) : 0;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
         if (lane == 0) {
-            atomicAdd(A.stats, (unsigned long long)pairs);
+            atomicAdd(A.stats, (unsigned long long)(long long)pairs);
             atomicAdd(A.stats + 2, (unsigned long long)cands * 32ull);
         }
     }
@@ -1621,8 +1753,16 @@ __global__ void __launch_bounds__(kWarps * 32, JT_CELL_MINB) k_walk_cell(CellArg
 
 int jt_cell_scan_blocks(int64_t ncells) { return (int)((ncells + kScanB - 1) / kScanB); }
 
+// Batches up to this many, two waves of the 148 x 28 resident warps, are split
+// among the warps of a block: a batch is a chain of ~1000 candidates, and
+// few of them leave the SMs waiting (2 x 16^3 particles, 292 batches: 49 us
+// whole, 24 us split; 2 x 32^3, 2217 batches: 78 against 73 us).  Larger
+// passes fill the SMs with whole batches and save the repeated setup (600,581
+// particles, 19,400 batches: 452 us whole, 515 us split).
+constexpr int64_t kCellSplitMax = 8192;
+
 int jt_b_cells(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t* d_pprefix, int nseg,
-               int64_t npart, const int64_t* d_cprefix, int nbox, int64_t ncells, const jt_cell_bufs& cb,
+               int64_t npart, int nbox, int64_t ncells, int64_t nslots, const jt_cell_bufs& cb,
                int order, int ngrid, int parts, float kick_frac, unsigned long long* stats,
                unsigned* d_err, cudaStream_t st, cudaEvent_t ev_walk0, cudaEvent_t ev_walk1, bool screened,
                const float4* pmacc, bool count_pairs)
@@ -1638,8 +1778,6 @@ int jt_b_cells(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_
     A.boxes = d_boxes;
     A.pprefix = d_pprefix;
     A.nseg = nseg;
-    A.nbox = nbox;
-    A.cprefix = d_cprefix;
     A.cb = cb;
     A.parts = parts;
     A.kick_frac = kick_frac;
@@ -1650,23 +1788,36 @@ int jt_b_cells(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_
     const unsigned gp = (unsigned)((npart + 255) / 256);
     if (ncells > 0 && cudaMemsetAsync(cb.ccount, 0, sizeof(int) * (size_t)ncells, st) != cudaSuccess)
         return JT_ECUDA;
+    if (nslots > 0 && cudaMemsetAsync(cb.cmap, 0xff, sizeof(int2) * (size_t)nslots, st) != cudaSuccess)
+        return JT_ECUDA;
+    if (ncells > 0 && cudaMemsetAsync(cb.reach, 0, sizeof(unsigned long long) * (size_t)nbox, st) != cudaSuccess)
+        return JT_ECUDA;
     if (cudaMemsetAsync(cb.segflag, 0, sizeof(int) * (size_t)nseg, st) != cudaSuccess) return JT_ECUDA;
     k_cell_key<<<gp, 256, 0, st>>>(A, npart);
     if (ncells == 0) cudaEventRecord(ev_walk1, st);
     if (ncells > 0) {
         const int nblk = jt_cell_scan_blocks(ncells);
-        k_scan_local<<<nblk, kScanB, 0, st>>>(cb.ccount, cb.cstart, ncells, cb.bsum);
-        k_scan_sums<<<1, kScanB, 0, st>>>(cb.bsum, nblk);
-        k_scan_add<<<nblk, kScanB, 0, st>>>(cb.cstart, ncells, cb.bsum, nblk);
+        k_scan_local<<<nblk, kScanT, 0, st>>>(cb.ccount, cb.cstart, ncells, cb.bsum);
+        k_scan_add<<<nblk, kScanT, 0, st>>>(cb.cstart, ncells, cb.bsum);
+        const int64_t nblocks = ncells / 8;
+        const int per = (int)std::min<int64_t>(32, std::max<int64_t>(1, nblocks / 8192));
+        const int64_t nw = (nblocks + per - 1) / per;
+        k_cell_dense<<<(unsigned)((nw + 7) / 8), 256, 0, st>>>(d_boxes, nbox, nblocks, per, cb);
         k_cell_scatter<<<gp, 256, 0, st>>>(A, npart);
-        const unsigned gw = (unsigned)((ncells + kWarps - 1) / kWarps);
+        const bool split = nslots <= kCellSplitMax;
+        const unsigned gw = (unsigned)(split ? nslots : (nslots + kWarps - 1) / kWarps);
         cudaEventRecord(ev_walk0, st);
-#define JT_CELL_LAUNCH(O, N)                                                                    \
+#define JT_CELL_LAUNCH3(O, N, SC, CN)                                                           \
     do {                                                                                        \
-        if (screened && count_pairs) k_walk_cell<O, N, true, true><<<gw, kWarps * 32, 0, st>>>(A, ncells);   \
-        else if (screened) k_walk_cell<O, N, true, false><<<gw, kWarps * 32, 0, st>>>(A, ncells);            \
-        else if (count_pairs) k_walk_cell<O, N, false, true><<<gw, kWarps * 32, 0, st>>>(A, ncells);         \
-        else k_walk_cell<O, N, false, false><<<gw, kWarps * 32, 0, st>>>(A, ncells);                         \
+        if (split) k_walk_cell<O, N, SC, CN, kWarps><<<gw, kWarps * 32, 0, st>>>(A, nslots);     \
+        else k_walk_cell<O, N, SC, CN, 1><<<gw, kWarps * 32, 0, st>>>(A, nslots);                \
+    } while (0)
+#define JT_CELL_LAUNCH(O, N)                                              \
+    do {                                                                  \
+        if (screened && count_pairs) JT_CELL_LAUNCH3(O, N, true, true);   \
+        else if (screened) JT_CELL_LAUNCH3(O, N, true, false);            \
+        else if (count_pairs) JT_CELL_LAUNCH3(O, N, false, true);         \
+        else JT_CELL_LAUNCH3(O, N, false, false);                         \
     } while (0)
         if (order == 4 && ngrid == 2) JT_CELL_LAUNCH(4, 2);
         else if (order == 4 && ngrid == 1) JT_CELL_LAUNCH(4, 1);
@@ -1676,6 +1827,7 @@ int jt_b_cells(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_
         else if (order == 2 && ngrid == 1) JT_CELL_LAUNCH(2, 1);
         else return JT_EINVAL;
 #undef JT_CELL_LAUNCH
+#undef JT_CELL_LAUNCH3
         cudaEventRecord(ev_walk1, st);
     }
     return cudaGetLastError() == cudaSuccess ? JT_OK : JT_ECUDA;
@@ -1713,7 +1865,7 @@ int jt_b_walk(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t
         else if (order == 2 && ngrid == 2) k_walk_acc<2, 2, 6, 32, true><<<g, kWarps * 32, 0, st>>>(A);
         else if (order == 2 && ngrid == 1) k_walk_acc<2, 1, 6, 32, true><<<g, kWarps * 32, 0, st>>>(A);
         else return JT_EINVAL;
-    } else if (order == 4 && ngrid == 2) launch_variant(pick_variant(g, ngroups, A, st), g, A, st);
+    } else if (order == 4 && ngrid == 2) launch_variant(pick_variant(ngroups), g, A, st);
     else if (order == 4 && ngrid == 1) k_walk_acc<4, 1, 6, 32, false><<<g, kWarps * 32, 0, st>>>(A);
     else if (order == 3 && ngrid == 2) k_walk_acc<3, 2, 6, 32, false><<<g, kWarps * 32, 0, st>>>(A);
     else if (order == 3 && ngrid == 1) k_walk_acc<3, 1, 6, 32, false><<<g, kWarps * 32, 0, st>>>(A);

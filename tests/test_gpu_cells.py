@@ -1,0 +1,133 @@
+"""The near-field cell walk against an FP64 sum over every pair inside the cut.
+
+Sizes and shapes where the batches of 32, the columns and the routing can go
+wrong: a few particles, counts around a batch, boxes of three cuts, sparse
+columns whose batches span the box, passes split among a block's warps and
+whole ones, clumps that stay in the cell walk and clumps that go to the tree
+walk, and several boxes (one without a cell grid) in one pass.
+"""
+import math
+import os
+import sys
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+sys.path.insert(0, os.path.join(ROOT, "janus-sim_b200"))
+
+
+def _erfc(x):
+    return np.vectorize(math.erfc)(x)
+
+
+def _short(pos, q, targets, L, r_s, rc, eps):
+    """(force, sum of |pair force|, what pairs within 1e-5 of the cut carry)."""
+    out, mag, edge = [], [], []
+    for t in targets:
+        d = pos - pos[t]
+        d -= L * np.round(d / L)
+        r2 = (d * d).sum(1)
+        near = (r2 > 0) & (r2 < (rc * 1.00001) ** 2)
+        d, r2, qj = d[near], r2[near], q[near]
+        rp = np.sqrt(r2 + eps * eps)
+        x = rp / (2 * r_s)
+        f = np.sign(q[t]) * qj * (_erfc(x) + 2 / math.sqrt(math.pi) * x * np.exp(-x * x)) / rp ** 3 if len(x) else x
+        r = np.sqrt(r2)
+        at_cut = r > rc * 0.99999
+        out.append((f[~at_cut, None] * d[~at_cut]).sum(0) if len(x) else np.zeros(3))
+        mag.append((np.abs(f) * r).sum())
+        edge.append((np.abs(f) * r)[at_cut].sum())
+    return np.array(out), np.array(mag), np.array(edge)
+
+
+def _points(kind, n, L, seed):
+    rng = np.random.default_rng(seed)
+    if kind == "uniform":
+        x = (rng.random((n, 3)) - 0.5) * L
+    elif kind == "line":       # one row of columns holds everything
+        x = np.stack([(rng.random(n) - 0.5) * L, rng.normal(0.0, 0.01 * L, n), rng.normal(0.0, 0.01 * L, n)], 1)
+    else:                      # a clump across the box's corner and a background
+        c = rng.normal(0.0, 0.02 * L, (n - n // 4, 3)) + 0.5 * L
+        x = np.concatenate([c, (rng.random((n // 4, 3)) - 0.5) * L])
+    return (np.remainder(x + 0.5 * L, L) - 0.5 * L).clip(-0.49999 * L, 0.49999 * L).astype(np.float32)
+
+
+# kind, n+, n-, L, PM grid, r_cut in units of r_s, theta
+CASES = [
+    ("uniform", 1, 0, 10.0, 16, 2.0, 0.5),
+    ("uniform", 3, 2, 10.0, 16, 2.0, 0.5),
+    ("uniform", 17, 15, 10.0, 16, 2.5, 0.5),
+    ("uniform", 17, 16, 10.0, 16, 2.5, 0.5),
+    ("uniform", 1500, 1301, 20.0, 16, 4.26, 0.5),       # just three cuts along the box
+    ("uniform", 0, 5000, 50.0, 32, 4.5, 0.5),
+    ("line", 700, 900, 40.0, 32, 4.5, 0.5),
+    ("uniform", 150000, 160001, 80.0, 128, 4.5, 0.5),   # more batches than are split
+    ("clump", 3000, 3000, 40.0, 64, 4.5, 0.5),          # stays in the cell walk
+    ("clump", 90000, 90000, 40.0, 64, 4.5, 0.3),        # its dense blocks go to the tree walk
+]
+
+
+def _config(J, L, M, cut, theta, n):
+    r_s = 1.25 * L / M
+    return J.Config(box_L=L, pm_grid=M, theta=theta, softening=0.02 * L / max(n, 1) ** (1 / 3), r_s=r_s,
+                    r_cut=cut * r_s, mu=3.0, G_mass_plus=1.0)
+
+
+def _check(J, cfg, pp, pm, ap, am, multipoles, seed=0):
+    pos = np.concatenate([pp, pm]).astype(np.float64)
+    mm = cfg.mu * len(pp) / len(pm) if len(pp) and len(pm) else cfg.mu
+    q = np.concatenate([np.full(len(pp), 1.0), np.full(len(pm), -float(np.float32(mm)))])
+    acc = np.concatenate([ap, am]).astype(np.float64)
+    t = np.random.default_rng(seed).choice(len(pos), min(len(pos), 60), replace=False)
+    f, mag, edge = _short(pos, q, t, cfg.box_L, cfg.r_s, cfg.r_cut, cfg.softening)
+    err = np.linalg.norm(acc[t] - f, axis=1)
+    # each pair's table entry is within 1.4e-5 of its force, its sum's rounding
+    # within 1e-6 of the magnitudes, and a coordinate near L/2 carries 6e-8 of
+    # it into differences of neighbours (relative to the softening at worst)
+    bound = (2e-5 + 1e-7 * cfg.box_L / cfg.softening) * mag + edge
+    if multipoles:   # nodes of the tree walk at this theta, against the force itself
+        bound = bound + 5e-3 * np.linalg.norm(f, axis=1) + 1e-4 * np.median(mag)
+    assert np.all(np.isfinite(acc)) and np.all(err <= bound + 1e-30), (err / np.maximum(bound, 1e-30)).max()
+
+
+@pytest.mark.parametrize("kind,n_p,n_m,L,M,cut,theta", CASES)
+def test_short_range_force(kind, n_p, n_m, L, M, cut, theta):
+    import janus_treepm as J
+    cfg = _config(J, L, M, cut, theta, n_p + n_m)
+    pp, pm = _points(kind, n_p, L, 1), _points(kind, n_m, L, 2)
+    s = J.Solver(cfg)
+    s.set_state(pp, None, pm, None)
+    ap, am = s.accel_part(J.JT_PART_SHORT)
+    nodes = s.timings()["node_interactions"]
+    s.close()
+    assert (nodes > 0) == (kind == "clump" and n_p > 50000), nodes
+    _check(J, cfg, pp, pm, ap, am, nodes > 0)
+
+
+def test_boxes_of_every_route_in_one_pass():
+    """Boxes without a cell grid (r_cut > L / 3), small and clustered ones share
+    the pass's cell and batch tables."""
+    import janus_treepm as J
+    rows = [CASES[4], ("uniform", 300, 200, 8.0, 16, 2.4, 0.0), CASES[9], CASES[1], CASES[8]]
+    cfgs = [_config(J, L, M, cut, th, n_p + n_m) for _, n_p, n_m, L, M, cut, th in rows]
+    cfgs[1].r_cut = 0.4 * cfgs[1].box_L
+    B = J.Batch()
+    pts = [(_points(k, n_p, L, 1), _points(k, n_m, L, 2)) for k, n_p, n_m, L, *_ in rows]
+    ids = [B.add(c, pp, None, pm, None) for c, (pp, pm) in zip(cfgs, pts)]
+    B.forces(ids, J.JT_PART_SHORT)
+    B.forces(ids)                      # the second pass meets the first one's tables
+    full = [B.accel(i) for i in ids]
+    B.forces(ids, J.JT_PART_PM)
+    B.close()
+    for c, (pp, pm), (ap, am) in zip(cfgs, pts, full):
+        s = J.Solver(c)
+        s.set_state(pp, None, pm, None)
+        rp, rm = s.accel()
+        s.close()
+        for a, r in ((ap, rp), (am, rm)):
+            if len(r):
+                rms = max(float(np.sqrt((r.astype(np.float64) ** 2).sum(1).mean())), 1e-30)
+                assert np.abs(a - r).max() <= 2e-5 * max(rms, float(np.abs(r).max()))
