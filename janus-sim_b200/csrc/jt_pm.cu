@@ -165,6 +165,105 @@ __global__ void k_b_tile_ranges(const jt_seg_dev* __restrict__ segs, const jt_bo
     if (t + 1 == (uint32_t)B.ntiles) r[2 * t].y = n;
 }
 
+// 1.5 * 2^23: x + kRound holds round(x) in its low bits
+constexpr float kRound = 12582912.0f;
+constexpr int kRoundBits = 0x4B400000;
+
+// A crowded tile's particles (a clump: many per cell), one at a time by whole
+// warps: lane (a, b, c) = (lane & 3, lane >> 2 & 3, lane >> 4) adds the
+// stencil's nodes x = a, y = b, z = c and c + 2.  A row step moves 24 banks and
+// a plane step 4 (the padded pitch), so the 32 atomics of an instruction go to
+// 32 banks, wherever the particle lies and whatever its neighbours do.  (One
+// particle per lane met up to 32 lanes in one cell inside a clump.)  The
+// stencils of 8 particles are computed first, one lane per particle and axis,
+// and left in the warp's scratch as the 16 products wx wy and the z weights
+// times the charge.  Deposit stage of clustered data: 2 x 64^3 particles
+// 0.73 -> 0.23 ms, 2 x 128^3 1.49 -> 0.63 ms.
+constexpr int kDepWarps = 16;
+// Tiles of more particles than this are crowded: half a particle per cell of
+// 16^3 and up, where the lanes of a warp begin to share cells.
+constexpr int kDepCrowded = 2048;
+constexpr int kDepRow = 24;   // words per particle: 16 products, two float4 (z weights, base, used)
+
+template <int ORDER, int NG>
+__device__ __forceinline__ void deposit_crowded(int* __restrict__ tile, float* __restrict__ ws_all,
+                                                const float4* __restrict__ pos0, const float4* __restrict__ pos1,
+                                                int n0, int ntot, float qs0, float qs1, float q0, float q1,
+                                                float halfL, float hinv, int ax, int by, int bz, int S, int W, int SW,
+                                                float* __restrict__ rho, int M)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float* ws = ws_all + warp * (8 * kDepRow);
+    const int la = lane & 3, lb = (lane >> 2) & 3, lc = lane >> 4;
+    const bool node = la < ORDER && lb < ORDER;
+    int* nodep = tile + lc * SW + lb * W + la;
+    const int mask = M - 1;
+    const int64_t G = (int64_t)M * M * M;
+    for (int k0 = warp * 8; k0 < ntot; k0 += kDepWarps * 8) {
+        const int k = k0 + (lane >> 2);
+        const bool valid = k < ntot;
+        const float4* pp = k < n0 ? pos0 + k : pos1 + (k - n0);
+        const float x = valid ? reinterpret_cast<const float*>(pp)[la] : 0.f;
+        const float qq = k < n0 ? qs0 : qs1;
+#pragma unroll
+        for (int g = 0; g < NG; g++) {
+            const float sh = 0.5f * g;
+            float w[4] = {0.f, 0.f, 0.f, 0.f};
+            const int l = jt_stencil<ORDER>((x + halfL) * hinv - sh, w) - (la == 0 ? ax : (la == 1 ? by : bz));
+            const unsigned bad = __ballot_sync(0xffffffffu, la < 3 && !(l >= 0 && l + ORDER <= (la == 0 ? W : S)));
+            const bool in = ((bad >> (lane & 28)) & 7u) == 0u;
+            const int lx = __shfl_sync(0xffffffffu, l, lane & 28), ly = __shfl_sync(0xffffffffu, l, (lane & 28) + 1),
+                      lz = __shfl_sync(0xffffffffu, l, (lane & 28) + 2);
+            const bool use = valid && in;
+            const int base = g * S * SW + lz * SW + ly * W + lx;
+            float* row = ws + (lane >> 2) * kDepRow;
+            float4* row4 = reinterpret_cast<float4*>(row);
+            __syncwarp();   // the previous particles' weights have been read
+            row4[la] = make_float4(w[0], w[1], w[2], w[3]);
+            __syncwarp();
+            const float4 wx = row4[0], wz = row4[2];
+            const float wy = row[4 + la];
+            __syncwarp();
+            row4[la] = make_float4(wx.x * wy, wx.y * wy, wx.z * wy, wx.w * wy);
+            if (la < 2) {
+                const float z0 = la == 0 ? wz.x : wz.y, z1 = la == 0 ? wz.z : wz.w;
+                row4[4 + la] = make_float4(qq * z0, qq * z1, __int_as_float(base), use ? 1.f : 0.f);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int p = 0; p < 8; p++) {
+                const float wxy = ws[p * kDepRow + 4 * lb + la];
+                const float4 z = reinterpret_cast<const float4*>(ws + p * kDepRow)[4 + lc];
+                if (node && z.w != 0.f) {
+                    int* at = nodep + __float_as_int(z.z);
+                    atomicAdd(at, __float_as_int(fmaf(wxy, z.x, kRound)) - kRoundBits);
+                    if (ORDER == 4 || lc + 2 < ORDER)
+                        atomicAdd(at + 2 * SW, __float_as_int(fmaf(wxy, z.y, kRound)) - kRoundBits);
+                }
+            }
+            if (valid && !in && la == 0) {
+                // outside the tile's halo: straight to the grid
+                const float4 p = *pp;
+                const float qg = k < n0 ? q0 : q1;
+                float ex[4], ey[4], ez[4];
+                const int ix = jt_stencil<ORDER>((p.x + halfL) * hinv - sh, ex);
+                const int iy = jt_stencil<ORDER>((p.y + halfL) * hinv - sh, ey);
+                const int iz = jt_stencil<ORDER>((p.z + halfL) * hinv - sh, ez);
+                float* gb = rho + g * G;
+#pragma unroll
+                for (int c = 0; c < ORDER; c++)
+#pragma unroll
+                    for (int bb = 0; bb < ORDER; bb++) {
+                        const float wyz = qg * ez[c] * ey[bb];
+                        const int64_t r = ((int64_t)((iz + c) & mask) * M + ((iy + bb) & mask)) * M;
+#pragma unroll
+                        for (int e = 0; e < ORDER; e++) atomicAdd(gb + r + ((ix + e) & mask), wyz * ex[e]);
+                    }
+            }
+        }
+    }
+}
+
 // Tiled deposit: one CTA per Morton-aligned tile of T^3 cells of one box.
 // The tile's particles are one contiguous range of each species' sorted
 // array (B.ranges); they are accumulated into a shared-memory copy of the
@@ -240,19 +339,13 @@ k_b_deposit(const jt_seg_dev* __restrict__ segs, const jt_box_dev* __restrict__ 
     const float4* pos0 = B.seg[0] >= 0 ? segs[B.seg[0]].pos : nullptr;
     const float4* pos1 = B.seg[1] >= 0 ? segs[B.seg[1]].pos : nullptr;
     float* rho = src ? B.rho_s : B.rho;
-    constexpr float kRound = 12582912.0f;   // 1.5 * 2^23: x + kRound holds round(x) in its low bits
-    constexpr int kRoundBits = 0x4B400000;
     __syncthreads();
-    // A crowded tile (a clump: many particles per cell) gives each thread a
-    // run of consecutive particles, so that the lanes of a warp, whose
-    // atomics meet in one instruction, sit far apart in the tile instead of
-    // in the same few cells; integer sums do not depend on the order
     const int ntot = n0 + n1, tid = (int)threadIdx.x, nth = (int)blockDim.x;
-    const int per = ntot > 2048 ? (ntot + nth - 1) / nth : 0;
-    const int niter = per ? per : (ntot - tid + nth - 1) / nth;
-    for (int i = 0; i < niter; i++) {
-        const int k = per ? tid * per + i : tid + i * nth;
-        if (k >= ntot) break;   // per > 0: the rest of this thread's run is past the end
+    const bool crowded = ntot > kDepCrowded;
+    if (crowded)
+        deposit_crowded<ORDER, NG>(tile, reinterpret_cast<float*>(tile4 + NG * S * SW4), pos0 + r.x, pos1 + r.z, n0,
+                                   ntot, qs0, qs1, q0, q1, halfL, hinv, ax, by, bz, S, W, SW, rho, M);
+    for (int k = crowded ? ntot : tid; k < ntot; k += nth) {
         float4 p;
         float qq, qg;
         if (k < n0) { p = pos0[r.x + k]; qq = qs0; qg = q0; } else { p = pos1[r.z + k - n0]; qq = qs1; qg = q1; }
@@ -596,11 +689,12 @@ int jt_b_deposit(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int6
 {
     if (ntiles <= 0) return JT_OK;
     int S = T + (order == 4 ? 4 : 3), W = T + 8;
-    size_t smem = sizeof(float) * (size_t)ngrid * S * (S * W + 4);   // padded plane pitch (k_b_deposit)
+    // padded plane pitch (k_b_deposit), then the warps' scratch
+    size_t smem = sizeof(float) * ((size_t)ngrid * S * (S * W + 4) + kDepWarps * 8 * kDepRow);
     // T16: every box of the pass has the tile edge 16 (T is the largest)
 #define JT_BDEP1(O, NG, TT)                                                                   \
     do {                                                                                      \
-        if (jt_smem_attr((const void*)k_b_deposit<O, NG, TT>, 96 * 1024) != JT_OK)            \
+        if (jt_smem_attr((const void*)k_b_deposit<O, NG, TT>, 104 * 1024) != JT_OK)            \
             return JT_ECUDA;                                                                  \
         k_b_deposit<O, NG, TT><<<(unsigned)ntiles, 512, smem, st>>>(d_segs, d_boxes, d_tprefix, nbox, src); \
     } while (0)
