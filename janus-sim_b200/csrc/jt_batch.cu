@@ -722,7 +722,7 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
         JT_TRY(B->cmap.ensure((size_t)(P.npart / 32 + P.ncols + 1), &grew));
         JT_TRY(B->csegflag.ensure((size_t)std::max<int>(nseg, 1), &grew));
     }
-    if (!P.screened) JT_TRY(B->pmacc.ensure((size_t)B->ngrid * std::max<int64_t>(P.npart, 1), &grew));
+    JT_TRY(B->pmacc.ensure((size_t)(P.screened ? 2 : 1) * B->ngrid * std::max<int64_t>(P.npart, 1), &grew));
 
     if (grew) B->gen++;
     std::vector<unsigned char> buf;
@@ -811,7 +811,7 @@ int tune_cells(jt_batch* B, Plan& P, int nseg, int parts, const float4* pmacc, b
         int flag[2] = {0, 0};
         unsigned long long reach = 0;
         for (int rep = 0; rep < 2 && r == JT_OK; rep++) {
-            r = jt_b_cells(P.d_post, P.d_bx, P.d_pp, nseg, P.npart, 1, P.ncells, P.npart / 32 + P.ncols, cb, B->order,
+            r = jt_b_cells(P.d_post, P.d_bx, P.d_pp, nseg, P.npart, 1, P.ncells, P.npart / 32 + P.ncols, cb,
                            B->ngrid, parts, 0.0f, nullptr, B->d_err, st, e0, e1, false, pmacc, false);
             if (r == JT_OK && (cudaMemcpyAsync(flag, B->csegflag.p, sizeof(int) * (size_t)nseg,
                                                cudaMemcpyDeviceToHost, st) != cudaSuccess ||
@@ -880,9 +880,8 @@ int force_pass(jt_batch* B, Plan& P, int parts, float kick_frac)
     }
     jt_b_tile_ranges(P.d_post, P.d_bx, P.d_ptp, nbox, P.npmtiles, st);
     const bool t16 = P.minT == 16 && P.maxT == 16;
-    JT_TRY(jt_b_deposit(P.d_post, P.d_bx, P.d_ptp, nbox, P.npmtiles, B->order, B->ngrid, P.maxT, st, 0, t16));
-    if (P.screened)
-        JT_TRY(jt_b_deposit(P.d_post, P.d_bx, P.d_ptp, nbox, P.npmtiles, B->order, B->ngrid, P.maxT, st, 1, t16));
+    const int nsrc = P.screened ? 2 : 1;   // the unsigned source of screened boxes
+    JT_TRY(jt_b_deposit(P.d_post, P.d_bx, P.d_ptp, nbox, P.npmtiles, B->order, B->ngrid, P.maxT, st, nsrc, t16));
     cudaEventRecord(B->ev[3], st);
     for (auto& kv : P.nslots) {
         Bucket& K = B->buckets[kv.first];
@@ -899,12 +898,11 @@ int force_pass(jt_batch* B, Plan& P, int parts, float kick_frac)
         JT_TRY(exec_c2r(K, kv.second, B->ngrid));
     }
     cudaEventRecord(B->ev[6], st);
-    // PM interpolation of every particle from shared-memory tiles (a pass with
-    // a screened box interpolates inside the walks: it has two sets of grids)
+    // PM interpolation of every particle from shared-memory tiles
     const float4* pmacc = nullptr;
-    if (!P.screened && (parts & JT_PART_PM) && P.npart > 0) {
+    if ((parts & JT_PART_PM) && P.npart > 0) {
         JT_TRY(jt_b_interp(P.d_post, P.d_bx, P.d_ptp, P.d_pp, nbox, P.npmtiles, B->order, B->ngrid, P.maxT,
-                           P.npart, B->pmacc.p, st, t16));
+                           P.npart, B->pmacc.p, st, nsrc, t16));
         pmacc = B->pmacc.p;
         B->tm.launches += 1;
     }
@@ -932,19 +930,19 @@ int force_pass(jt_batch* B, Plan& P, int parts, float kick_frac)
                            B->tflag.p, B->cdense.p, B->creach.p, B->cmap.p, B->csegflag.p};
         if (!done)
             JT_TRY(jt_b_cells(P.d_post, P.d_bx, P.d_pp, nseg, P.npart, nbox, P.ncells,
-                              P.ncells > 0 ? P.npart / 32 + P.ncols : 0, cb, B->order, B->ngrid, parts, kick_frac,
+                              P.ncells > 0 ? P.npart / 32 + P.ncols : 0, cb, B->ngrid, parts, kick_frac,
                               B->d_stats, B->d_err, st, B->ev[8], B->ev[9], P.screened, pmacc, B->counters));
         tflag = B->tflag.p;
         jt_b_build_trees(P.d_post, P.d_bx, nseg, P.d_ip, P.ninternal, P.d_pp, P.npart, st, B->csegflag.p);
         B->tm.launches += P.npart > 0 ? (P.ncells > 0 ? 6 : 1) : 0;
     }
-    JT_TRY(jt_b_walk(P.d_post, P.d_bx, P.d_gp, nseg, P.ngroups, pool, B->order, B->ngrid, parts,
+    JT_TRY(jt_b_walk(P.d_post, P.d_bx, P.d_gp, nseg, P.ngroups, pool, B->ngrid, parts,
                      kick_frac, B->d_stats, B->d_err, st, P.d_pp, tflag, P.screened,
                      tflag ? B->csegflag.p : nullptr, pmacc, P.npart));
     cudaEventRecord(B->ev[7], st);
     B->pending = true;
     B->tm.launches += (P.npart > 0 ? 8 : 0) + (P.ninternal > 0 ? 1 : 0) + (P.npart > 0 ? 1 : 0) +
-                      (P.npmtiles > 0 ? (P.screened ? 3 : 2) : 0) + (P.nmodes > 0 ? 1 : 0) +
+                      (P.npmtiles > 0 ? 2 : 0) + (P.nmodes > 0 ? 1 : 0) +
                       (P.nztiles > 0 ? (P.screened ? 2 : 1) * ((P.zsizes & 1) + ((P.zsizes >> 1) & 1)) : 0) +
                       (P.ngroups > 0 ? 1 : 0);
     for (int id : P.ids) {

@@ -298,12 +298,11 @@ int jt_pm_tile_edge(int M);
 // batched PM stages (jt_pm.cu)
 void jt_b_tile_ranges(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t* d_tprefix,
                       int nbox, int64_t ntiles, cudaStream_t st);
-// src 0: the signed source D = sum s m W into B.rho; src 1: the unsigned
-// source S = sum m W into B.rho_s (boxes without rho_s skip the pass).
+// Source 0, the signed D = sum s m W, goes into B.rho; with nsrc 2 source 1,
+// the unsigned S = sum m W, into B.rho_s of the boxes that have it.
 // T: the largest tile edge of the pass; T16: every box's tile edge is 16.
 int jt_b_deposit(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t* d_tprefix,
-                 int nbox, int64_t ntiles, int order, int ngrid, int T, cudaStream_t st, int src = 0,
-                 bool T16 = false);
+                 int nbox, int64_t ntiles, int order, int ngrid, int T, cudaStream_t st, int nsrc, bool T16);
 // The fused z transforms + k-space of 512^3 and 256^3 grids whose planes
 // cuFFT transforms in 2D (jt_zfft.cu): CTAs per box (0 for other grid
 // sizes), and the launches over every such box of a pass (sizes: bit 0 if
@@ -314,13 +313,13 @@ int jt_b_zfft_kspace(const jt_box_dev* d_boxes, const int64_t* d_zprefix, int nb
                      int k_min, int src, int sizes, cudaStream_t st);
 void jt_b_kspace(const jt_box_dev* d_boxes, const int64_t* d_kprefix, int nbox, int64_t nmodes,
                  int interlace, int k_min, cudaStream_t st);
-// PM interpolation of every particle of the pass from each interlaced grid
-// (tiles staged in shared memory): pmacc[b * npart + i], i = pprefix[seg] +
-// index, the force of grid b on a unit m+ particle.  T: the largest tile edge
-// of the pass (every box's T <= it; region (T + 4)^3 x 3 floats).
+// PM interpolation of every particle of the pass from each interlaced grid of
+// each source (tiles staged in shared memory): pmacc[q * npart + i], i =
+// pprefix[seg] + index, q = source * ngrid + grid: the force of that grid on a
+// unit m+ particle.  T: the largest tile edge of the pass (every box's T <= it).
 int jt_b_interp(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t* d_tprefix,
                 const int64_t* d_pprefix, int nbox, int64_t ntiles, int order, int ngrid, int T,
-                int64_t npart, float4* pmacc, cudaStream_t st, bool T16 = false);
+                int64_t npart, float4* pmacc, cudaStream_t st, int nsrc, bool T16);
 
 // walk (jt_walk.cu)
 struct jt_walk_params {
@@ -333,10 +332,6 @@ struct jt_walk_params {
     float slack;        // candidate prefilter: padding of the group's box
     float rc2_keep;     // candidate prefilter: widened cut
     float mass[2];      // per-species particle mass (G folded in) times c^3
-    int M;
-    float h_inv;        // M / L
-    int order;          // PM assignment order (2 CIC, 3 TSC)
-    int ngrid;          // PM grids (2 with interlacing)
     int parts;          // JT_PART_* bits: 1 = PM, 2 = tree
 };
 // Batched accurate walk over every segment's 32-particle groups (gprefix);
@@ -345,7 +340,7 @@ struct jt_walk_params {
 // stats[0] pair interactions inside r_cut, [1] node (multipole) interactions,
 // [2] candidate particles distance-tested
 int jt_b_walk(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t* d_gprefix, int nseg,
-              int64_t ngroups, const jt_tree_dev& pool, int order, int ngrid, int parts,
+              int64_t ngroups, const jt_tree_dev& pool, int ngrid, int parts,
               float kick_frac, unsigned long long* stats, unsigned* d_err, cudaStream_t st,
               const int64_t* d_pprefix = nullptr, const unsigned char* tflag = nullptr,
               bool screened = false, const int* segflag = nullptr, const float4* pmacc = nullptr,
@@ -368,7 +363,7 @@ struct jt_cell_bufs {
 };
 int jt_b_cells(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t* d_pprefix, int nseg,
                int64_t npart, int nbox, int64_t ncells, int64_t nslots, const jt_cell_bufs& cb,
-               int order, int ngrid, int parts, float kick_frac, unsigned long long* stats,
+               int ngrid, int parts, float kick_frac, unsigned long long* stats,
                unsigned* d_err, cudaStream_t st, cudaEvent_t ev_walk0, cudaEvent_t ev_walk1,
                bool screened = false, const float4* pmacc = nullptr, bool count_pairs = true);
 int jt_cell_scan_blocks(int64_t ncells);

@@ -297,11 +297,12 @@ __device__ __forceinline__ void deposit_crowded(int* __restrict__ tile, float* _
 template <int ORDER, int NG, int TT>
 __global__ void __launch_bounds__(512, 2)
 k_b_deposit(const jt_seg_dev* __restrict__ segs, const jt_box_dev* __restrict__ boxes,
-            const int64_t* __restrict__ tprefix, int nbox, int src)
+            const int64_t* __restrict__ tprefix, int nbox)
 {
     extern __shared__ int4 tile4[];
     int* tile = reinterpret_cast<int*>(tile4);
     const int64_t q = blockIdx.x;
+    const int src = blockIdx.y;   // 1: the unsigned source of screened boxes
     const int b = jt_find(tprefix, nbox, q);
     const jt_box_dev& B = boxes[b];
     if (src && !B.rho_s) return;   // the unsigned source of an unscreened box: not used
@@ -400,7 +401,7 @@ k_b_deposit(const jt_seg_dev* __restrict__ segs, const jt_box_dev* __restrict__ 
 }
 
 // PM interpolation, tiled like the deposit: one CTA per (Morton tile of T^3
-// cells of one box, interlaced grid b).  The three force grids of grid b
+// cells of one box, interlaced grid b of one source).  The three force grids of it
 // over the tile plus its stencil halo, nodes T t - 2 .. T t + T + 1 on every
 // axis (R = T + 4, the reach of CIC, TSC and PCS stencils of a particle in
 // the tile, the interlaced grid's half-cell shift included), are staged in
@@ -417,9 +418,13 @@ k_b_deposit(const jt_seg_dev* __restrict__ segs, const jt_box_dev* __restrict__ 
 // against 4.77 ms at 2x224^3; 16 lanes, one per (x, y) column, measured
 // slower still (0.90 against 0.68 ms at 2x112^3).  A particle whose stencil leaves
 // the region (outside its tile by the Morton key's rounding) reads the grid.
-// Output: pmacc[b * npart + i] = the interpolated force of grid b on a unit
-// m+ particle (i = the particle's index in the pass, pprefix[seg] + index);
-// the walks average the grids and apply the sign.
+// Output: pmacc[q * npart + i] = the interpolated force of grid set q on a unit
+// m+ particle (i = the particle's index in the pass, pprefix[seg] + index; q =
+// the interlaced grid, plus ngrid for the unsigned source of a screened box);
+// the walks average the grids and apply the signs.  (Screened passes used to
+// interpolate in the walks' epilogue, one lane per particle reading its 768
+// scattered nodes: 2x64^3 particles, PM 128^3, two sources: cell walk 0.87 ->
+// 0.41 ms for 0.20 ms here.)
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem)
 {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -450,10 +455,10 @@ k_b_interp(const jt_seg_dev* __restrict__ segs, const jt_box_dev* __restrict__ b
     float2* reg2 = reinterpret_cast<float2*>(reg4);
     const float* reg = reinterpret_cast<const float*>(reg4);
     const int64_t q = blockIdx.x;
-    const int g = blockIdx.y;   // interlaced grid
     const int b = jt_find(tprefix, nbox, q);
     const jt_box_dev& B = boxes[b];
-    if (g >= B.ngrid) return;
+    const int src = (int)blockIdx.y / B.ngrid, g = (int)blockIdx.y % B.ngrid;   // source, interlaced grid
+    if (src && !B.force_s) return;   // the unsigned source of an unscreened box
     const uint32_t t = (uint32_t)(q - tprefix[b]);
     const int4 r = B.ranges[t];
     const int n0 = r.y - r.x, n1 = r.w - r.z;
@@ -463,7 +468,7 @@ k_b_interp(const jt_seg_dev* __restrict__ segs, const jt_box_dev* __restrict__ b
     const int oy = (int)compact3(t >> 1) * T - 2;
     const int oz = (int)compact3(t >> 2) * T - 2;
     const int64_t G = (int64_t)M * M * M;
-    const float* __restrict__ F = B.force + (int64_t)g * 3 * G;
+    const float* __restrict__ F = (src ? B.force_s : B.force) + (int64_t)g * 3 * G;
     const int rows = 3 * R * R;
     if (TT == 16) {
         float* regw = reinterpret_cast<float*>(reg4);
@@ -495,7 +500,7 @@ k_b_interp(const jt_seg_dev* __restrict__ segs, const jt_box_dev* __restrict__ b
     const float4* pos1 = B.seg[1] >= 0 ? segs[B.seg[1]].pos : nullptr;
     const int64_t base0 = B.seg[0] >= 0 ? pprefix[B.seg[0]] : 0;
     const int64_t base1 = B.seg[1] >= 0 ? pprefix[B.seg[1]] : 0;
-    float4* __restrict__ out = pmacc + (int64_t)g * npart;
+    float4* __restrict__ out = pmacc + (int64_t)blockIdx.y * npart;
     const int RR = R * R, RRR = RR * R;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     const int gl = lane & 3;            // lane in the particle's group: x offset of the stencil
@@ -685,9 +690,10 @@ void jt_b_tile_ranges(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const
 
 // all boxes of a batch share order, ngrid and the tile edge T
 int jt_b_deposit(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t* d_tprefix,
-                 int nbox, int64_t ntiles, int order, int ngrid, int T, cudaStream_t st, int src, bool T16)
+                 int nbox, int64_t ntiles, int order, int ngrid, int T, cudaStream_t st, int nsrc, bool T16)
 {
     if (ntiles <= 0) return JT_OK;
+    const dim3 grid((unsigned)ntiles, (unsigned)nsrc);
     int S = T + (order == 4 ? 4 : 3), W = T + 8;
     // padded plane pitch (k_b_deposit), then the warps' scratch
     size_t smem = sizeof(float) * ((size_t)ngrid * S * (S * W + 4) + kDepWarps * 8 * kDepRow);
@@ -696,7 +702,7 @@ int jt_b_deposit(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int6
     do {                                                                                      \
         if (jt_smem_attr((const void*)k_b_deposit<O, NG, TT>, 104 * 1024) != JT_OK)            \
             return JT_ECUDA;                                                                  \
-        k_b_deposit<O, NG, TT><<<(unsigned)ntiles, 512, smem, st>>>(d_segs, d_boxes, d_tprefix, nbox, src); \
+        k_b_deposit<O, NG, TT><<<grid, 512, smem, st>>>(d_segs, d_boxes, d_tprefix, nbox);    \
     } while (0)
 #define JT_BDEP(O, NG)                    \
     do {                                  \
@@ -717,13 +723,13 @@ int jt_b_deposit(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int6
 
 int jt_b_interp(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t* d_tprefix,
                 const int64_t* d_pprefix, int nbox, int64_t ntiles, int order, int ngrid, int T,
-                int64_t npart, float4* pmacc, cudaStream_t st, bool T16)
+                int64_t npart, float4* pmacc, cudaStream_t st, int nsrc, bool T16)
 {
     if (ntiles <= 0 || npart <= 0) return JT_OK;
     const int R = T + 4;
     const size_t smem = sizeof(float) * 3 * (size_t)R * R * R;
     if (smem > 200 * 1024) return JT_EINVAL;
-    dim3 grid((unsigned)ntiles, (unsigned)ngrid);
+    const dim3 grid((unsigned)ntiles, (unsigned)(ngrid * nsrc));
 #define JT_INTERP1(O, TT)                                                                              \
     do {                                                                                              \
         if (jt_smem_attr((const void*)k_b_interp<O, TT>, (int)smem) != JT_OK) return JT_ECUDA;        \

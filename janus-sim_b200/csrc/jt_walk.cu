@@ -1,4 +1,4 @@
-// Short-range tree walk (+ PM interpolation, + kick), and the step kernels.
+// Short-range walks (+ kick), and the step kernels.
 //
 // ACCURATE walk (k_walk_acc): one warp per group of 32 Morton-consecutive
 // target particles of one species; both species' trees are walked in the same
@@ -11,8 +11,8 @@
 // Accepted entries are compacted with ballots into shared-memory lists that
 // all 32 lanes evaluate against their own particle once 32 entries are
 // queued.  Far-field (node) sums are Kahan-compensated.  The PM acceleration
-// is interpolated first (CIC of the three force grids) and the kick is
-// applied in the epilogue, so acc is written once.
+// (jt_b_interp) is added and the kick applied in the epilogue, so acc is
+// written once.
 //
 // Pair force (G folded into m):  a_i += s_i s_j m_j S(r_p) r / r_p^3 for
 // |r| < r_cut, r_p^2 = r^2 + eps^2, S(x) = erfc(x) + 2x/sqrt(pi) e^{-x^2},
@@ -436,7 +436,7 @@ __device__ __forceinline__ void drain_ranges(WalkWarpSmem& S, int nr, int& nc,
 // SCR: the pass holds a screened box; the other species' tree of a screened
 // box is walked with the Yukawa table and without multipoles (their
 // expansion is of the Newtonian kernel), i.e. every pair inside r_cut
-template <int ORDER, int NG, bool WRAP, int BKT, bool SCR>
+template <bool WRAP, int BKT, bool SCR>
 __device__ __forceinline__ void walk_trees(const WalkArgs& A, const jt_box_dev& B,
                                            const jt_walk_params& P, WalkWarpSmem& S, int s, int lane,
                                            const float4& p, bool valid, float gcx, float gcy,
@@ -621,53 +621,11 @@ __device__ __forceinline__ void walk_trees(const WalkArgs& A, const jt_box_dev& 
     }
 }
 
-// PM acceleration of a unit m+ particle at p from one set of force grids
-// (SG false, B.force: the signed source's, which an m- particle takes with
-// minus sign; SG true, B.force_s: the unsigned source's of a screened box,
-// taken by both): the deposit's stencil on every grid (the interlaced grid's
-// nodes sit half a cell higher), averaged over the grids
-template <int ORDER, int NG, bool SG = false>
-__device__ __forceinline__ Acc3 pm_interp(const jt_box_dev& B, const float4& p)
-{
-    Acc3 pm = {0.f, 0.f, 0.f};
-    {
-        const int M = B.M, mask = M - 1;
-        const int64_t G = (int64_t)M * M * M;
-        const float gx = (p.x + B.halfL) * B.h_inv, gy = (p.y + B.halfL) * B.h_inv,
-                    gz = (p.z + B.halfL) * B.h_inv;
-#pragma unroll
-        for (int b = 0; b < NG; b++) {
-            const float sh = 0.5f * b;
-            float wx[ORDER], wy[ORDER], wz[ORDER];
-            const int ix = jt_stencil<ORDER>(gx - sh, wx);
-            const int iy = jt_stencil<ORDER>(gy - sh, wy);
-            const int iz = jt_stencil<ORDER>(gz - sh, wz);
-            const float* __restrict__ F = (SG ? B.force_s : B.force) + (int64_t)b * 3 * G;
-#pragma unroll
-            for (int c = 0; c < ORDER; c++)
-#pragma unroll
-                for (int bb = 0; bb < ORDER; bb++) {
-                    const float wyz = wz[c] * wy[bb];
-                    const int64_t row = ((int64_t)((iz + c) & mask) * M + ((iy + bb) & mask)) * M;
-#pragma unroll
-                    for (int a = 0; a < ORDER; a++) {
-                        const int64_t id = row + ((ix + a) & mask);
-                        const float w = wyz * wx[a];
-                        pm.x += w * __ldg(F + id);
-                        pm.y += w * __ldg(F + G + id);
-                        pm.z += w * __ldg(F + 2 * G + id);
-                    }
-                }
-        }
-        if (NG == 2) { pm.x *= 0.5f; pm.y *= 0.5f; pm.z *= 0.5f; }
-    }
-
-    return pm;
-}
-
-// The PM acceleration of a unit m+ particle computed by the tiled
-// interpolation kernel (jt_b_interp) for pass particle gi: the mean of the
-// interlaced grids' values.
+// The PM acceleration of a unit m+ particle from one source's grids, computed
+// by the tiled interpolation kernel (jt_b_interp) for pass particle gi: the
+// mean of the interlaced grids' values.  The signed source's sets come first
+// (an m- particle takes their mean with minus sign), then the unsigned
+// source's of screened boxes (taken by both).
 template <int NG>
 __device__ __forceinline__ Acc3 pm_from_tiles(const float4* __restrict__ pmacc, int64_t npart, int64_t gi)
 {
@@ -684,7 +642,7 @@ __device__ __forceinline__ Acc3 pm_from_tiles(const float4* __restrict__ pmacc, 
 // MINB: resident blocks per SM the register budget is sized for (6 -> 80
 // registers); BKT: nodes with <= BKT particles are streamed as ranges
 // (<= 32: one lane per particle when a range is loaded)
-template <int ORDER, int NG, int MINB, int BKT, bool SCR>
+template <int NG, int MINB, int BKT, bool SCR>
 __global__ void __launch_bounds__(kWarps * 32, MINB) k_walk_acc(WalkArgs A)
 {
     static_assert(BKT <= 32, "a range is loaded one particle per lane");
@@ -715,7 +673,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_walk_acc(WalkArgs A)
     // box, 1e-5 relative on the cut
     P.slack = B.halfL * 9.5367431640625e-7f;
     P.rc2_keep = B.rc2 * 1.00001f;
-    P.M = B.M; P.h_inv = B.h_inv; P.order = ORDER; P.ngrid = NG; P.parts = A.parts;
+    P.parts = A.parts;
     const int64_t ns = SG.n;
     const int64_t i = grp * 32 + lane;
     const bool valid = i < ns;
@@ -732,7 +690,6 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_walk_acc(WalkArgs A)
     float ghx = 0.5f * (hix - lox), ghy = 0.5f * (hiy - loy), ghz = 0.5f * (hiz - loz);
 
     Acc3 pm = {0.f, 0.f, 0.f};
-    if (SCR && (P.parts & 1)) pm = pm_interp<ORDER, NG>(B, p);   // no tile interpolation in a screened pass
 
     Acc3 near = {0.f, 0.f, 0.f}, far = {0.f, 0.f, 0.f}, comp = {0.f, 0.f, 0.f};
     unsigned pairs = 0, nodes = 0, cands = 0;   // per lane (warp totals < 2^32)
@@ -740,19 +697,19 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_walk_acc(WalkArgs A)
     // groups wider than L/8 take the minimum image per pair
     const bool wide = fmaxf(fmaxf(ghx, ghy), ghz) > 0.125f * P.L;
     if (wide)
-        walk_trees<ORDER, NG, true, BKT, SCR>(A, B, P, S, s, lane, p, valid, gcx, gcy, gcz, ghx, ghy, ghz, near,
+        walk_trees<true, BKT, SCR>(A, B, P, S, s, lane, p, valid, gcx, gcy, gcz, ghx, ghy, ghz, near,
                                     far, comp, pairs, nodes, cands, wc);
     else
-        walk_trees<ORDER, NG, false, BKT, SCR>(A, B, P, S, s, lane, p, valid, gcx, gcy, gcz, ghx, ghy, ghz, near,
+        walk_trees<false, BKT, SCR>(A, B, P, S, s, lane, p, valid, gcx, gcy, gcz, ghx, ghy, ghz, near,
                                      far, comp, pairs, nodes, cands, wc);
 
     if (valid && mine) {
-        if (!SCR && (P.parts & 1)) pm = pm_from_tiles<NG>(A.pmacc, A.npart, A.pprefix[g] + i);
+        if (P.parts & 1) pm = pm_from_tiles<NG>(A.pmacc, A.npart, A.pprefix[g] + i);
         float ax = sgn_s * pm.x + near.x + (far.x - comp.x);
         float ay = sgn_s * pm.y + near.y + (far.y - comp.y);
         float az = sgn_s * pm.z + near.z + (far.z - comp.z);
         if (SCR && B.force_s && (P.parts & 1)) {
-            const Acc3 ps = pm_interp<ORDER, NG, true>(B, p);
+            const Acc3 ps = pm_from_tiles<NG>(A.pmacc + NG * A.npart, A.npart, A.pprefix[g] + i);
             ax += ps.x;
             ay += ps.y;
             az += ps.z;
@@ -1125,13 +1082,13 @@ struct WalkVariant {
 constexpr WalkVariant kVariants[] = {{6, 32}, {5, 32}, {6, 24}};
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 
-// the variants of the default PM scheme (PCS, interlaced)
+// the variants of the interlaced PM scheme
 void launch_variant(int v, unsigned g, const WalkArgs& A, cudaStream_t st)
 {
     switch (v) {
-    case 1: k_walk_acc<4, 2, 5, 32, false><<<g, kWarps * 32, 0, st>>>(A); break;
-    case 2: k_walk_acc<4, 2, 6, 24, false><<<g, kWarps * 32, 0, st>>>(A); break;
-    default: k_walk_acc<4, 2, 6, 32, false><<<g, kWarps * 32, 0, st>>>(A); break;
+    case 1: k_walk_acc<2, 5, 32, false><<<g, kWarps * 32, 0, st>>>(A); break;
+    case 2: k_walk_acc<2, 6, 24, false><<<g, kWarps * 32, 0, st>>>(A); break;
+    default: k_walk_acc<2, 6, 32, false><<<g, kWarps * 32, 0, st>>>(A); break;
     }
 }
 
@@ -1533,7 +1490,7 @@ __device__ __forceinline__ unsigned cell_chunk(const CellWarpSmem& S, int cnt, C
 // less than 8 (64: 0.66 ms)
 constexpr int kCellMinBlocks = 7;
 // SPLIT: the warps that share a batch (1, or the block's kWarps)
-template <int ORDER, int NG, bool SCR, bool CNT, int SPLIT>
+template <int NG, bool SCR, bool CNT, int SPLIT>
 __global__ void __launch_bounds__(kWarps * 32, kCellMinBlocks) k_walk_cell(CellArgs A, int64_t nslots)
 {
     __shared__ CellWarpSmem smem_all[kWarps];
@@ -1708,14 +1665,11 @@ __global__ void __launch_bounds__(kWarps * 32, kCellMinBlocks) k_walk_cell(CellA
     const bool valid = t == t0 + lane;   // its own target
     if (valid && part == 0) {
         Acc3 pm = {0.f, 0.f, 0.f};
-        const float4 p = A.cb.cpos[t];
-        // a pass with a screened box has no tile interpolation
-        if (A.parts & 1)
-            pm = SCR ? pm_interp<ORDER, NG>(B, p) : pm_from_tiles<NG>(A.pmacc, A.npart, A.pprefix[id.x] + id.y);
+        if (A.parts & 1) pm = pm_from_tiles<NG>(A.pmacc, A.npart, A.pprefix[id.x] + id.y);
         const jt_seg_dev& SG = A.segs[id.x];
         float ax = si * pm.x + near.x, ay = si * pm.y + near.y, az = si * pm.z + near.z;
         if (SCR && B.force_s && (A.parts & 1)) {
-            const Acc3 ps = pm_interp<ORDER, NG, true>(B, p);
+            const Acc3 ps = pm_from_tiles<NG>(A.pmacc + NG * A.npart, A.npart, A.pprefix[id.x] + id.y);
             ax += ps.x;
             ay += ps.y;
             az += ps.z;
@@ -1763,7 +1717,7 @@ constexpr int64_t kCellSplitMax = 8192;
 
 int jt_b_cells(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t* d_pprefix, int nseg,
                int64_t npart, int nbox, int64_t ncells, int64_t nslots, const jt_cell_bufs& cb,
-               int order, int ngrid, int parts, float kick_frac, unsigned long long* stats,
+               int ngrid, int parts, float kick_frac, unsigned long long* stats,
                unsigned* d_err, cudaStream_t st, cudaEvent_t ev_walk0, cudaEvent_t ev_walk1, bool screened,
                const float4* pmacc, bool count_pairs)
 {
@@ -1807,34 +1761,29 @@ int jt_b_cells(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_
         const bool split = nslots <= kCellSplitMax;
         const unsigned gw = (unsigned)(split ? nslots : (nslots + kWarps - 1) / kWarps);
         cudaEventRecord(ev_walk0, st);
-#define JT_CELL_LAUNCH3(O, N, SC, CN)                                                           \
+#define JT_CELL_LAUNCH2(N, SC, CN)                                                              \
     do {                                                                                        \
-        if (split) k_walk_cell<O, N, SC, CN, kWarps><<<gw, kWarps * 32, 0, st>>>(A, nslots);     \
-        else k_walk_cell<O, N, SC, CN, 1><<<gw, kWarps * 32, 0, st>>>(A, nslots);                \
+        if (split) k_walk_cell<N, SC, CN, kWarps><<<gw, kWarps * 32, 0, st>>>(A, nslots);        \
+        else k_walk_cell<N, SC, CN, 1><<<gw, kWarps * 32, 0, st>>>(A, nslots);                   \
     } while (0)
-#define JT_CELL_LAUNCH(O, N)                                              \
-    do {                                                                  \
-        if (screened && count_pairs) JT_CELL_LAUNCH3(O, N, true, true);   \
-        else if (screened) JT_CELL_LAUNCH3(O, N, true, false);            \
-        else if (count_pairs) JT_CELL_LAUNCH3(O, N, false, true);         \
-        else JT_CELL_LAUNCH3(O, N, false, false);                         \
+#define JT_CELL_LAUNCH(N)                                              \
+    do {                                                               \
+        if (screened && count_pairs) JT_CELL_LAUNCH2(N, true, true);   \
+        else if (screened) JT_CELL_LAUNCH2(N, true, false);            \
+        else if (count_pairs) JT_CELL_LAUNCH2(N, false, true);         \
+        else JT_CELL_LAUNCH2(N, false, false);                         \
     } while (0)
-        if (order == 4 && ngrid == 2) JT_CELL_LAUNCH(4, 2);
-        else if (order == 4 && ngrid == 1) JT_CELL_LAUNCH(4, 1);
-        else if (order == 3 && ngrid == 2) JT_CELL_LAUNCH(3, 2);
-        else if (order == 3 && ngrid == 1) JT_CELL_LAUNCH(3, 1);
-        else if (order == 2 && ngrid == 2) JT_CELL_LAUNCH(2, 2);
-        else if (order == 2 && ngrid == 1) JT_CELL_LAUNCH(2, 1);
-        else return JT_EINVAL;
+        if (ngrid == 2) JT_CELL_LAUNCH(2);
+        else JT_CELL_LAUNCH(1);
 #undef JT_CELL_LAUNCH
-#undef JT_CELL_LAUNCH3
+#undef JT_CELL_LAUNCH2
         cudaEventRecord(ev_walk1, st);
     }
     return cudaGetLastError() == cudaSuccess ? JT_OK : JT_ECUDA;
 }
 
 int jt_b_walk(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t* d_gprefix, int nseg,
-              int64_t ngroups, const jt_tree_dev& pool, int order, int ngrid, int parts,
+              int64_t ngroups, const jt_tree_dev& pool, int ngrid, int parts,
               float kick_frac, unsigned long long* stats, unsigned* d_err, cudaStream_t st,
               const int64_t* d_pprefix, const unsigned char* tflag, bool screened, const int* segflag,
               const float4* pmacc, int64_t npart)
@@ -1858,20 +1807,13 @@ int jt_b_walk(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t
     A.segflag = tflag ? segflag : nullptr;
     unsigned g = (unsigned)((ngroups + kWarps - 1) / kWarps);
     if (screened) {
-        if (order == 4 && ngrid == 2) k_walk_acc<4, 2, 6, 32, true><<<g, kWarps * 32, 0, st>>>(A);
-        else if (order == 4 && ngrid == 1) k_walk_acc<4, 1, 6, 32, true><<<g, kWarps * 32, 0, st>>>(A);
-        else if (order == 3 && ngrid == 2) k_walk_acc<3, 2, 6, 32, true><<<g, kWarps * 32, 0, st>>>(A);
-        else if (order == 3 && ngrid == 1) k_walk_acc<3, 1, 6, 32, true><<<g, kWarps * 32, 0, st>>>(A);
-        else if (order == 2 && ngrid == 2) k_walk_acc<2, 2, 6, 32, true><<<g, kWarps * 32, 0, st>>>(A);
-        else if (order == 2 && ngrid == 1) k_walk_acc<2, 1, 6, 32, true><<<g, kWarps * 32, 0, st>>>(A);
-        else return JT_EINVAL;
-    } else if (order == 4 && ngrid == 2) launch_variant(pick_variant(ngroups), g, A, st);
-    else if (order == 4 && ngrid == 1) k_walk_acc<4, 1, 6, 32, false><<<g, kWarps * 32, 0, st>>>(A);
-    else if (order == 3 && ngrid == 2) k_walk_acc<3, 2, 6, 32, false><<<g, kWarps * 32, 0, st>>>(A);
-    else if (order == 3 && ngrid == 1) k_walk_acc<3, 1, 6, 32, false><<<g, kWarps * 32, 0, st>>>(A);
-    else if (order == 2 && ngrid == 2) k_walk_acc<2, 2, 6, 32, false><<<g, kWarps * 32, 0, st>>>(A);
-    else if (order == 2 && ngrid == 1) k_walk_acc<2, 1, 6, 32, false><<<g, kWarps * 32, 0, st>>>(A);
-    else return JT_EINVAL;
+        if (ngrid == 2) k_walk_acc<2, 6, 32, true><<<g, kWarps * 32, 0, st>>>(A);
+        else k_walk_acc<1, 6, 32, true><<<g, kWarps * 32, 0, st>>>(A);
+    } else if (ngrid == 2) {
+        launch_variant(pick_variant(ngroups), g, A, st);
+    } else {
+        k_walk_acc<1, 6, 32, false><<<g, kWarps * 32, 0, st>>>(A);
+    }
     return cudaGetLastError() == cudaSuccess ? JT_OK : JT_ECUDA;
 }
 
