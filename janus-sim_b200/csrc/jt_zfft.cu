@@ -369,15 +369,18 @@ __device__ __forceinline__ void zfft_body(const jt_box_dev& B, const float2* __r
         }
         P[i] = keep ? make_float2(z.x * green, z.y * green) : make_float2(0.f, 0.f);
     }
-    // the six force spectra (three components, times the interlaced grid's
-    // phase for the second grid), each transformed back along z
+    // The force spectra -i k_c phi, times the interlaced grid's phase for the
+    // second grid, transformed back along z.  k_x and k_y are constant along a
+    // column, so the x and y components are both multiples of phi's transform:
+    // two transforms per grid (phi and k_z phi) instead of three (2.11 -> 1.92 ms
+    // on a 512^3 grid pair, 0.244 -> 0.212 ms on 256^3).
 #pragma unroll 1
-    for (int s = 0; s < 3 * (IL ? 2 : 1); s++) {
-        const int c = s % 3, g = s / 3;
+    for (int s = 0; s < 2 * (IL ? 2 : 1); s++) {
+        const int c = s & 1, g = s >> 1;
 #pragma unroll
         for (int i = 0; i < 8; i++) {
             const int kz = kz_of<M>(t, i);
-            const float dd = c == 0 ? ax.y : (c == 1 ? ay.y : __ldg(&ta[kz]).y);
+            const float dd = c == 0 ? 1.0f : __ldg(&ta[kz]).y;
             float2 f = make_float2(dd * P[i].y, -dd * P[i].x);
             if (g == 1) {
                 const float4 bz = __ldg(&tb[kz]);
@@ -389,9 +392,17 @@ __device__ __forceinline__ void zfft_body(const jt_box_dev& B, const float2* __r
         if constexpr (M == 512) fft512_inv(v, XA, XB, tw1, tw2, t);
         else fft256_inv(v, XA, XB, tw1, tw2, t);
         if (colok) {
-            float2* o = out + (int64_t)s * Gc + cb;
+            float2* o = out + (int64_t)(3 * g + (c ? 2 : 0)) * Gc + cb;
+            if (c) {
 #pragma unroll
-            for (int j = 0; j < 8; j++) o[(t + T * j) * sz] = v[j];
+                for (int j = 0; j < 8; j++) o[(t + T * j) * sz] = v[j];
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; j++) o[(t + T * j) * sz] = make_float2(ax.y * v[j].x, ax.y * v[j].y);
+                o += Gc;
+#pragma unroll
+                for (int j = 0; j < 8; j++) o[(t + T * j) * sz] = make_float2(ay.y * v[j].x, ay.y * v[j].y);
+            }
         }
     }
 }
