@@ -173,8 +173,7 @@ struct Bucket {                 // PM scratch of the boxes with grid M in a pass
 size_t grid_bytes(int64_t M, int ngrid)
 {
     int64_t G = M * M * M, Gc = M * M * (M / 2 + 1);
-    int T = jt_pm_tile_edge((int)M);
-    int64_t nt = (M / T) * (M / T) * (M / T);
+    int64_t nt = M <= 32 ? M * M * M / 512 : M * M * M / 4096;   // PM tiles (max_tiles)
     return (size_t)(ngrid * (G * 4 + Gc * 8) + 3 * ngrid * (Gc * 8 + G * 4) + nt * 16);
 }
 
@@ -330,9 +329,23 @@ void box_release(jt_box_state* b)
     b->kappa = 0.0;
 }
 
-int tile_shift_of(int M)
+// PM tiles of 16^3 cells; a pass of few of them (its grids' sum at most
+// kSmallTiles) takes 8^3 tiles, so that the deposit and the interpolation, one
+// CTA per tile, reach more SMs: 2 x 16^3 particles, PM 32^3 (8 tiles): deposit
+// stage 28 -> 20 us, interpolation 23 -> 10 us.  Larger passes keep 16^3, whose
+// halo is smaller (PM 64^3, 64 tiles: 31 against 28 us and 25 against 28).
+constexpr int64_t kSmallTiles = 32;
+
+int64_t tiles_of(int M, int T) { return (int64_t)(M / T) * (M / T) * (M / T); }
+// the most tiles a pass may cut a grid into
+int64_t max_tiles(int M)
 {
-    int T = jt_pm_tile_edge(M);
+    const int T = jt_pm_tile_edge(M);
+    return T > 8 && tiles_of(M, T) <= kSmallTiles ? tiles_of(M, 8) : tiles_of(M, T);
+}
+
+int tile_shift_of(int M, int T)
+{
     int W = 1024 / M * T;  // tile edge in Morton cells (power of two)
     int lw = 0;
     while ((1 << lw) < W) lw++;
@@ -399,8 +412,7 @@ int bucket_ensure(jt_batch* B, Bucket& k, int M, int count)
     const int64_t G = (int64_t)M * M * M, Gc = (int64_t)M * M * (M / 2 + 1);
     if (count > k.cap) {
         B->gen++;
-        int T = jt_pm_tile_edge(M);
-        int64_t nt = (int64_t)(M / T) * (M / T) * (M / T);
+        const int64_t nt = max_tiles(M);
         const int add = count - k.cap;
         BucketChunk c;
         c.slots = add;
@@ -513,6 +525,13 @@ int cell_columns(double L, double rcut, int64_t n)
     return q >= 256.0 ? 256 : (q < 1.0 ? 1 : (int)q);
 }
 
+// the share of a uniform box's particles that a block has in reach (k_cell_dense)
+double uniform_reach(const jt_box_dev& d)
+{
+    const double w = 2 * d.colm + 1, nb = d.nb;
+    return std::min(1.0, w * w * std::min(w, nb) / (nb * nb * nb));
+}
+
 // the cell list of a box with nb columns per axis
 void box_cells(jt_box_dev& d, int64_t n, int nb, const jt_config& c, double rcut)
 {
@@ -527,6 +546,7 @@ void box_cells(jt_box_dev& d, int64_t n, int nb, const jt_config& c, double rcut
     const double bin = L / nb * (L / nb) * (L / d.nbx);
     d.cell_dmax = (float)(JT_CELL_KMAX / (27.0 * c.r_cut * c.r_cut * c.r_cut) * bin);
     d.reach_max = (float)(JT_CELL_REACH / c.theta * (double)n);   // theta 0: no multipoles, never
+    d.reach_raw = (float)(1.3 * (double)n * (double)n * uniform_reach(d));
 }
 
 // Size the scratch pools for the listed boxes, lay out their segments and
@@ -590,6 +610,9 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
     P.ptprefix.push_back(0); P.kprefix.push_back(0); P.zprefix.push_back(0);
     P.cells = cells_enabled();
     P.bx.resize(nb);
+    int64_t tiles16 = 0;
+    for (int k = 0; k < nb; k++) tiles16 += tiles_of(B->boxes[ids[k]]->M, jt_pm_tile_edge(B->boxes[ids[k]]->M));
+    const bool small = tiles16 <= kSmallTiles;
     for (int k = 0; k < nb; k++) {
         jt_box_state* b = B->boxes[ids[k]];
         const jt_config& c = b->cfg;
@@ -612,9 +635,9 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
         d.M = M;
         d.order = b->order;
         d.ngrid = b->ngrid;
-        d.T = jt_pm_tile_edge(M);
-        d.tile_shift = tile_shift_of(M);
-        d.ntiles = (M / d.T) * (M / d.T) * (M / d.T);
+        d.T = small ? std::min(8, jt_pm_tile_edge(M)) : jt_pm_tile_edge(M);
+        d.tile_shift = tile_shift_of(M, d.T);
+        d.ntiles = (int)tiles_of(M, d.T);
         P.maxT = std::max(P.maxT, d.T);
         P.minT = std::min(P.minT, d.T);
         Bucket& K = B->buckets[M];
@@ -627,7 +650,7 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
         d.force_k = C.force_k + (size_t)qi * 3 * b->ngrid * Gc;
         d.force = C.force + (size_t)qi * 3 * b->ngrid * G;
         d.tabs = b->tabs;
-        d.ranges = C.ranges + (size_t)qi * d.ntiles;
+        d.ranges = C.ranges + (size_t)qi * max_tiles(M);
         // the deposit flushes its tiles with 16-byte reductions
         if (reinterpret_cast<uintptr_t>(d.rho) & 15) return JT_ECUDA;
         if (b->ytab) {
@@ -825,9 +848,8 @@ int tune_cells(jt_batch* B, Plan& P, int nseg, int parts, const float4* pmacc, b
             // crowded or clustered at the default already (the mean number of
             // particles in reach twice that of a uniform box): keep it
             if (r == JT_OK && nb == nmax) {
-                const double w = 2 * d.colm + 1, n = (double)(bs->n[0] + bs->n[1]);
-                const double uniform = std::min(1.0, w * w * std::min(w, (double)nb) / ((double)nb * nb * nb));
-                crowded = flag[0] || flag[1] || (double)reach > 2.0 * n * n * uniform;
+                const double n = (double)(bs->n[0] + bs->n[1]);
+                crowded = flag[0] || flag[1] || (double)reach > 2.0 * n * n * uniform_reach(d);
                 if (crowded) break;
             }
         }
@@ -879,9 +901,9 @@ int force_pass(jt_batch* B, Plan& P, int parts, float kick_frac)
         }
     }
     jt_b_tile_ranges(P.d_post, P.d_bx, P.d_ptp, nbox, P.npmtiles, st);
-    const bool t16 = P.minT == 16 && P.maxT == 16;
+    const int tile = P.minT == P.maxT && (P.maxT == 16 || P.maxT == 8) ? P.maxT : 0;
     const int nsrc = P.screened ? 2 : 1;   // the unsigned source of screened boxes
-    JT_TRY(jt_b_deposit(P.d_post, P.d_bx, P.d_ptp, nbox, P.npmtiles, B->order, B->ngrid, P.maxT, st, nsrc, t16));
+    JT_TRY(jt_b_deposit(P.d_post, P.d_bx, P.d_ptp, nbox, P.npmtiles, B->order, B->ngrid, P.maxT, st, nsrc, tile));
     cudaEventRecord(B->ev[3], st);
     for (auto& kv : P.nslots) {
         Bucket& K = B->buckets[kv.first];
@@ -902,7 +924,7 @@ int force_pass(jt_batch* B, Plan& P, int parts, float kick_frac)
     const float4* pmacc = nullptr;
     if ((parts & JT_PART_PM) && P.npart > 0) {
         JT_TRY(jt_b_interp(P.d_post, P.d_bx, P.d_ptp, P.d_pp, nbox, P.npmtiles, B->order, B->ngrid, P.maxT,
-                           P.npart, B->pmacc.p, st, nsrc, t16));
+                           P.npart, B->pmacc.p, st, nsrc, tile));
         pmacc = B->pmacc.p;
         B->tm.launches += 1;
     }

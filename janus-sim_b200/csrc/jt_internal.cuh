@@ -121,6 +121,7 @@ struct jt_box_dev {
     float reach_max;      // the box's sum of particles in reach above which dense blocks go to the tree walk
     float cell_inv;       // nb / L
     float cellx_inv;      // nbx / L
+    float reach_raw;      // ... above which the cell walk takes differences of unscaled positions
     int64_t cbase;        // this box's first cell in the pass's cell tables
     int64_t colbase;      // this box's first column in the pass
 };
@@ -300,9 +301,10 @@ void jt_b_tile_ranges(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const
                       int nbox, int64_t ntiles, cudaStream_t st);
 // Source 0, the signed D = sum s m W, goes into B.rho; with nsrc 2 source 1,
 // the unsigned S = sum m W, into B.rho_s of the boxes that have it.
-// T: the largest tile edge of the pass; T16: every box's tile edge is 16.
+// T: the largest tile edge of the pass; TT: every box's tile edge (16 or 8), or
+// 0 when they differ.
 int jt_b_deposit(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t* d_tprefix,
-                 int nbox, int64_t ntiles, int order, int ngrid, int T, cudaStream_t st, int nsrc, bool T16);
+                 int nbox, int64_t ntiles, int order, int ngrid, int T, cudaStream_t st, int nsrc, int TT);
 // The fused z transforms + k-space of 512^3 and 256^3 grids whose planes
 // cuFFT transforms in 2D (jt_zfft.cu): CTAs per box (0 for other grid
 // sizes), and the launches over every such box of a pass (sizes: bit 0 if
@@ -319,7 +321,7 @@ void jt_b_kspace(const jt_box_dev* d_boxes, const int64_t* d_kprefix, int nbox, 
 // unit m+ particle.  T: the largest tile edge of the pass (every box's T <= it).
 int jt_b_interp(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t* d_tprefix,
                 const int64_t* d_pprefix, int nbox, int64_t ntiles, int order, int ngrid, int T,
-                int64_t npart, float4* pmacc, cudaStream_t st, int nsrc, bool T16);
+                int64_t npart, float4* pmacc, cudaStream_t st, int nsrc, int TT);
 
 // walk (jt_walk.cu)
 struct jt_walk_params {

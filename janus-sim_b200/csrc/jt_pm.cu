@@ -290,8 +290,8 @@ __device__ __forceinline__ void deposit_crowded(int* __restrict__ tile, float* _
 // the tile's bound that is 2^-30 (2^-23 of one particle's full weight in a
 // sparse tile), below the FP32 sums' own rounding of the densest cells.
 // Integer sums do not depend on the order of the atomics, so a tile's
-// values are reproducible.  TT: the tile edge as a constant (16, the edge of
-// every grid of 16^3 and up) or 0 (read per box).
+// values are reproducible.  TT: the tile edge as a constant (16, or 8 in small
+// passes) or 0 (read per box).
 // 512 threads, 2 blocks per SM (the 69 KB tile allows 3 of 256): 32 warps
 // per SM hide more of the shared-memory atomics' latency.
 template <int ORDER, int NG, int TT>
@@ -438,13 +438,13 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 
-// TT: the tile edge as a constant (16, every grid of 16^3 and up: the
-// region's index arithmetic folds) or 0 (read per box).  With TT = 16 a
-// staged row of 20 nodes is stored rotated, [16 nodes of the tile | 2 above
-// | 2 below], so that the tile's 16 nodes (64-byte aligned in the grid and
-// in the row) travel as four 16-byte copies and each halo as one 8-byte
-// copy: 6 copies per row instead of 10; node lx of the row sits at
-// (lx + 18) % 20.
+// TT: the tile edge as a constant (16, or 8 in small passes: the region's
+// index arithmetic folds) or 0 (read per box).  With a constant edge a staged
+// row of TT + 4 nodes is stored rotated, [TT nodes of the tile | 2 above | 2
+// below], so that the tile's nodes (32-byte aligned in the grid and 16-byte in
+// the row) travel as 16-byte copies and each halo as one 8-byte copy (6 copies
+// per row instead of 10 at 16); node lx of the row sits at (lx + TT + 2) %
+// (TT + 4).
 template <int ORDER, int TT>
 __global__ void __launch_bounds__(512, 2)
 k_b_interp(const jt_seg_dev* __restrict__ segs, const jt_box_dev* __restrict__ boxes,
@@ -470,17 +470,18 @@ k_b_interp(const jt_seg_dev* __restrict__ segs, const jt_box_dev* __restrict__ b
     const int64_t G = (int64_t)M * M * M;
     const float* __restrict__ F = (src ? B.force_s : B.force) + (int64_t)g * 3 * G;
     const int rows = 3 * R * R;
-    if (TT == 16) {
+    if (TT > 0) {
+        constexpr int kPieces = TT / 4 + 2;
         float* regw = reinterpret_cast<float*>(reg4);
-        for (int k = threadIdx.x; k < rows * 6; k += blockDim.x) {
-            const int piece = k % 6, row = k / 6;
+        for (int k = threadIdx.x; k < rows * kPieces; k += blockDim.x) {
+            const int piece = k % kPieces, row = k / kPieces;
             const int y = row % R, zc = row / R;
             const int z = zc % R, c = zc / R;
             const int64_t rb = c * G + ((int64_t)((oz + z) & mask) * M + ((oy + y) & mask)) * M;
             float* dst = regw + row * R;
-            if (piece < 4) cp_async16(dst + 4 * piece, F + rb + ox + 2 + 4 * piece);   // the tile's nodes
-            else if (piece == 4) cp_async8(dst + 16, F + rb + ((ox + 18) & mask));     // 2 above
-            else cp_async8(dst + 18, F + rb + (ox & mask));                            // 2 below
+            if (piece < TT / 4) cp_async16(dst + 4 * piece, F + rb + ox + 2 + 4 * piece);       // the tile's nodes
+            else if (piece == TT / 4) cp_async8(dst + TT, F + rb + ((ox + TT + 2) & mask));     // 2 above
+            else cp_async8(dst + TT + 2, F + rb + (ox & mask));                                 // 2 below
         }
     } else {
         // x pairs start at even nodes (ox and M even): 8-byte aligned, never split by the wrap
@@ -529,7 +530,7 @@ k_b_interp(const jt_seg_dev* __restrict__ segs, const jt_box_dev* __restrict__ b
             // then one weight along x
             if (in) {
                 const int xp = lx + gl;
-                const float* base = reg + (lz * R + ly) * R + (TT == 16 ? (xp >= 2 ? xp - 2 : xp + 18) : xp);
+                const float* base = reg + (lz * R + ly) * R + (TT > 0 ? (xp >= 2 ? xp - 2 : xp + TT + 2) : xp);
 #pragma unroll
                 for (int zz = 0; zz < ORDER; zz++) {
                     float bx = 0.f, by = 0.f, bz = 0.f;
@@ -690,24 +691,25 @@ void jt_b_tile_ranges(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const
 
 // all boxes of a batch share order, ngrid and the tile edge T
 int jt_b_deposit(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t* d_tprefix,
-                 int nbox, int64_t ntiles, int order, int ngrid, int T, cudaStream_t st, int nsrc, bool T16)
+                 int nbox, int64_t ntiles, int order, int ngrid, int T, cudaStream_t st, int nsrc, int TT)
 {
     if (ntiles <= 0) return JT_OK;
     const dim3 grid((unsigned)ntiles, (unsigned)nsrc);
     int S = T + (order == 4 ? 4 : 3), W = T + 8;
     // padded plane pitch (k_b_deposit), then the warps' scratch
     size_t smem = sizeof(float) * ((size_t)ngrid * S * (S * W + 4) + kDepWarps * 8 * kDepRow);
-    // T16: every box of the pass has the tile edge 16 (T is the largest)
-#define JT_BDEP1(O, NG, TT)                                                                   \
+    // TT: the tile edge of every box of the pass (16 or 8), or 0 (T is the largest)
+#define JT_BDEP1(O, NG, E)                                                                   \
     do {                                                                                      \
-        if (jt_smem_attr((const void*)k_b_deposit<O, NG, TT>, 104 * 1024) != JT_OK)            \
+        if (jt_smem_attr((const void*)k_b_deposit<O, NG, E>, 104 * 1024) != JT_OK)            \
             return JT_ECUDA;                                                                  \
-        k_b_deposit<O, NG, TT><<<grid, 512, smem, st>>>(d_segs, d_boxes, d_tprefix, nbox);    \
+        k_b_deposit<O, NG, E><<<grid, 512, smem, st>>>(d_segs, d_boxes, d_tprefix, nbox);    \
     } while (0)
 #define JT_BDEP(O, NG)                    \
     do {                                  \
-        if (T16) JT_BDEP1(O, NG, 16);     \
-        else JT_BDEP1(O, NG, 0);          \
+        if (TT == 16) JT_BDEP1(O, NG, 16);     \
+        else if (TT == 8) JT_BDEP1(O, NG, 8);  \
+        else JT_BDEP1(O, NG, 0);               \
     } while (0)
     if (order == 2 && ngrid == 1) JT_BDEP(2, 1);
     else if (order == 2 && ngrid == 2) JT_BDEP(2, 2);
@@ -723,22 +725,23 @@ int jt_b_deposit(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int6
 
 int jt_b_interp(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t* d_tprefix,
                 const int64_t* d_pprefix, int nbox, int64_t ntiles, int order, int ngrid, int T,
-                int64_t npart, float4* pmacc, cudaStream_t st, int nsrc, bool T16)
+                int64_t npart, float4* pmacc, cudaStream_t st, int nsrc, int TT)
 {
     if (ntiles <= 0 || npart <= 0) return JT_OK;
     const int R = T + 4;
     const size_t smem = sizeof(float) * 3 * (size_t)R * R * R;
     if (smem > 200 * 1024) return JT_EINVAL;
     const dim3 grid((unsigned)ntiles, (unsigned)(ngrid * nsrc));
-#define JT_INTERP1(O, TT)                                                                              \
+#define JT_INTERP1(O, E)                                                                              \
     do {                                                                                              \
-        if (jt_smem_attr((const void*)k_b_interp<O, TT>, (int)smem) != JT_OK) return JT_ECUDA;        \
-        k_b_interp<O, TT><<<grid, 512, smem, st>>>(d_segs, d_boxes, d_tprefix, d_pprefix, nbox, npart, pmacc); \
+        if (jt_smem_attr((const void*)k_b_interp<O, E>, (int)smem) != JT_OK) return JT_ECUDA;        \
+        k_b_interp<O, E><<<grid, 512, smem, st>>>(d_segs, d_boxes, d_tprefix, d_pprefix, nbox, npart, pmacc); \
     } while (0)
 #define JT_INTERP(O)                      \
     do {                                  \
-        if (T16) JT_INTERP1(O, 16);       \
-        else JT_INTERP1(O, 0);            \
+        if (TT == 16) JT_INTERP1(O, 16);       \
+        else if (TT == 8) JT_INTERP1(O, 8);    \
+        else JT_INTERP1(O, 0);                 \
     } while (0)
     if (order == 2) JT_INTERP(2);
     else if (order == 3) JT_INTERP(3);

@@ -1437,10 +1437,11 @@ __device__ __forceinline__ void ld_inside(float2& ab, const float2* __restrict__
 // CNT: count the lane's pairs inside the cut (the pair counters; one
 // instruction per candidate, off unless the caller asks for them).
 // y = r^2 c^2 + ye (c = 1 / (2 r_s), ye = eps^2 c^2), and the pair is inside
-// the cut for y < yc.  The differences are of the positions as they are
-// (scaling them by c when they are staged saves half a slot per candidate,
-// but its rounding, of the size of a coordinate's ulp, sets the error of
-// close pairs: 1e-5 of the force inside a clump against 1.5e-6).  No clamp on
+// the cut for y < yc.  Positions come scaled by c (T.c2 = 1) except in
+// clustered boxes (T.c2 = c^2), where the scaling's rounding, of the size of a
+// coordinate's ulp, would set the error of close pairs: 1e-5 of the force
+// inside a clump against 1.5e-6.  (A second loop without T.c2 for the scaled
+// boxes, half a slot per candidate less, measured no faster.)  No clamp on
 // the table index: the caller bounds ye >= 2^-32 and yc < 64, so that every
 // y of a lane inside the cut indexes the table ([2^-32, 2^6)); lanes outside
 // it load nothing.
@@ -1569,14 +1570,16 @@ __global__ void __launch_bounds__(kWarps * 32, kCellMinBlocks) k_walk_cell(CellA
         }
         __syncwarp();
         if ((A.parts & 2) && nr > 0) {
+            const bool raw = (float)A.cb.reach[where.x] > B.reach_raw;
+            const float ps = raw ? 1.0f : cc;   // what positions are scaled by
             const float ye = fmaxf(B.eps2 * c2, 2.3283064365386963e-10f);
             const float2* __restrict__ yt = (SCR && B.ytab) ? B.ytab : g_ltab;
             CellTarget T;
-            T.nx = pack2(-p.x, -p.x);
-            T.ny = pack2(-p.y, -p.y);
-            T.nz = pack2(-p.z, -p.z);
+            T.nx = pack2(-p.x * ps, -p.x * ps);
+            T.ny = pack2(-p.y * ps, -p.y * ps);
+            T.nz = pack2(-p.z * ps, -p.z * ps);
             T.ye = pack2(ye, ye);
-            T.c2 = pack2(c2, c2);
+            T.c2 = raw ? pack2(c2, c2) : pack2(1.0f, 1.0f);
             T.si = si;
             T.yc = fminf(fmaf(B.rc2, c2, ye), 64.0f * 0.99999f);
             T.ax = T.ay = T.az = 0.0f;
@@ -1603,9 +1606,9 @@ __global__ void __launch_bounds__(kWarps * 32, kCellMinBlocks) k_walk_cell(CellA
                 const unsigned km = __ballot_sync(0xffffffffu, keep);
                 if (keep) {
                     const int at = nc + __popc(km & lt);
-                    S.cx[at] = c.x;
-                    S.cy[at] = c.y;
-                    S.cz[at] = c.z;
+                    S.cx[at] = c.x * ps;
+                    S.cy[at] = c.y * ps;
+                    S.cz[at] = c.z * ps;
                     S.cq[at] = c.w;
                 }
                 nc += __popc(km);
@@ -1630,16 +1633,16 @@ __global__ void __launch_bounds__(kWarps * 32, kCellMinBlocks) k_walk_cell(CellA
             if (nc > 0) {
                 // pad to a multiple of 4 with points outside any cut (< L / 2)
                 if (lane < ((-nc) & 3)) {
-                    S.cx[nc + lane] = gcx + 4.0f * B.L;
-                    S.cy[nc + lane] = gcy;
-                    S.cz[nc + lane] = gcz;
+                    S.cx[nc + lane] = (gcx + 4.0f * B.L) * ps;
+                    S.cy[nc + lane] = gcy * ps;
+                    S.cz[nc + lane] = gcz * ps;
                     S.cq[nc + lane] = 0.0f;
                 }
                 __syncwarp();
                 hits += cell_chunk<SCR, CNT>(S, (nc + 3) & ~3, T, yt);
                 cands += nc;
             }
-            const float sc = si * c2 * cc;
+            const float sc = si * c2 * (raw ? cc : 1.0f);   // sum w d, d scaled by ps
             near = Acc3{T.ax * sc, T.ay * sc, T.az * sc};
         }
     }
