@@ -193,6 +193,7 @@ struct Plan {
     std::vector<int64_t> pprefix, iprefix, tprefix, gprefix, ptprefix, kprefix, zprefix;
     int64_t npart = 0, ninternal = 0, nsorttiles = 0, ngroups = 0, npmtiles = 0, nmodes = 0, ncells = 0;
     int64_t ncols = 0;                    // columns of the near-field cell lists
+    size_t o_cmap = 0, o_ccount = 0, o_segflag = 0, cellz_bytes = 0;   // layout of jt_batch::cellz
     int64_t nztiles = 0;                  // CTAs of the fused z-transform kernel
     int zsizes = 0;                       // its grid sizes in the pass: bit 0 512^3, bit 1 256^3
     bool cells = false;                   // the near-field cell walk runs (jt_b_cells)
@@ -233,27 +234,40 @@ struct jt_batch {
     Pool<int2> child, range;
     Pool<int> parent, flag;
     // near-field cell list (jt_b_cells)
-    Pool<int> ccount, cstart, cbsum, ccell, csegflag;
+    Pool<int> cstart, cbsum, ccell;
     Pool<unsigned> cslot;
     Pool<float4> cpos;
     Pool<float4> pmacc;                 // PM accelerations of the pass, per interlaced grid
-    Pool<int2> cid, cmap;
+    Pool<int2> cid;
     Pool<unsigned char> tflag, cdense;
-    Pool<unsigned long long> creach;
+    Pool<unsigned char> cellz;          // the cell list's arrays that start at zero (jt_cell_bufs.zero)
     Pool<float4> com, bmin, bmax, quad0;
     Pool<float2> quad1;
-    Pool<uint32_t> m30, vals, vals_alt, keys_alt, hist, status, tickets;
+    Pool<uint32_t> m30, vals, vals_alt, keys_alt;
+    Pool<uint32_t> sortz;               // the sort's words that start at zero: tickets, counts, look-back
     Pool<unsigned char> desc;           // device copy of the pass's tables
     unsigned char* hdesc = nullptr;     // pinned host staging of the tables
     size_t hdesc_cap = 0;
     cudaEvent_t desc_done = nullptr;    // the last upload from hdesc finished
     std::map<int, Bucket> buckets;
-    unsigned* d_err = nullptr;
+    // pair counters (8 words, never reset: the host keeps what it has read)
+    // and the error word behind them, read back together
     unsigned long long* d_stats = nullptr;
-    cudaEvent_t ev[11] = {};            // 8, 9: around the cell walk kernel; 6-10: interpolation
+    unsigned* d_err = nullptr;
+    unsigned long long* h_stats = nullptr;   // pinned
+    unsigned long long seen[8] = {};
+    // two sets of a pass's stage events, used in turn, so that the steps of
+    // one call queue up while the host reads the step before
+    // (8, 9: around the cell walk kernel; 6-10: interpolation; 11, 12: kick and drift)
+    struct Events {
+        cudaEvent_t e[13] = {};
+        bool pending = false;           // recorded, not yet added to the timings
+        bool kicked = false;            // 11, 12 too
+    } evs[2];
+    int evi = 0;
+    cudaEvent_t ev_call[2] = {};        // around a call
     bool counters = false;              // the cell walk counts its pairs (jt_batch_set_counters)
     bool cell_tune = true;              // tune_cells may run (jtb_set_cell_tune)
-    bool pending = false;               // a pass's events await jtb_finish
     jt_timings tm = {};
     int64_t phase[4] = {0, 0, 0, 0};
     Plan plan;
@@ -549,6 +563,8 @@ void box_cells(jt_box_dev& d, int64_t n, int nb, const jt_config& c, double rcut
     d.reach_raw = (float)(1.3 * (double)n * (double)n * uniform_reach(d));
 }
 
+constexpr size_t kTickets = 32;   // words before the sort's counts (one ticket per pass)
+
 // Size the scratch pools for the listed boxes, lay out their segments and
 // boxes, and upload every table in one copy.
 int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* steps, Plan& P)
@@ -578,9 +594,7 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
     JT_TRY(B->quad1.ensure(nodes, &grew));
     JT_TRY(B->m30.ensure(parts, &grew)); JT_TRY(B->vals.ensure(parts, &grew));
     JT_TRY(B->vals_alt.ensure(parts, &grew)); JT_TRY(B->keys_alt.ensure(parts, &grew));
-    JT_TRY(B->hist.ensure((size_t)nseg * 4 * 256, &grew));
-    JT_TRY(B->status.ensure((size_t)stiles * 4 * 256, &grew));
-    JT_TRY(B->tickets.ensure(4, &grew));
+    JT_TRY(B->sortz.ensure(kTickets + ((size_t)nseg + (size_t)stiles) * 4 * 256, &grew));
     for (int k = 0; k < nb; k++) P.by_M[B->boxes[ids[k]]->M].push_back(k);
     std::vector<int> slot(nb);
     for (auto& kv : P.by_M) {
@@ -699,8 +713,8 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
             g.vals = B->vals.p + o_part;
             g.vals_alt = B->vals_alt.p + o_part;
             g.keys_alt = B->keys_alt.p + o_part;
-            g.hist = B->hist.p + (size_t)P.pre.size() * 4 * 256;
-            g.status = B->status.p + (size_t)o_tile * 4 * 256;
+            g.hist = B->sortz.p + kTickets + (size_t)P.pre.size() * 4 * 256;
+            g.status = B->sortz.p + kTickets + ((size_t)nseg + (size_t)o_tile) * 4 * 256;
             d.seg[s] = (int)P.pre.size();
             jt_seg_dev pre = g, post = g;
             pre.pos = b->pos[s]; pre.vel = b->vel[s]; pre.acc = b->acc[s];
@@ -732,7 +746,6 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
     P.nmodes = P.kprefix.back();
     P.nztiles = P.zprefix.back();
     if (P.cells) {
-        JT_TRY(B->ccount.ensure((size_t)std::max<int64_t>(P.ncells, 1), &grew));
         JT_TRY(B->cstart.ensure((size_t)P.ncells + 1, &grew));
         JT_TRY(B->cbsum.ensure((size_t)jt_cell_scan_blocks(P.ncells) + 1, &grew));
         JT_TRY(B->ccell.ensure((size_t)std::max<int64_t>(P.npart, 1), &grew));
@@ -741,9 +754,13 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
         JT_TRY(B->cid.ensure((size_t)std::max<int64_t>(P.npart, 1), &grew));
         JT_TRY(B->tflag.ensure((size_t)std::max<int64_t>(P.npart, 1), &grew));
         JT_TRY(B->cdense.ensure((size_t)P.ncells / 8 + 1, &grew));
-        JT_TRY(B->creach.ensure((size_t)nb, &grew));
-        JT_TRY(B->cmap.ensure((size_t)(P.npart / 32 + P.ncols + 1), &grew));
-        JT_TRY(B->csegflag.ensure((size_t)std::max<int>(nseg, 1), &grew));
+        // reach (boxes), cmap (slots), ccount (cells), segflag (segments)
+        const size_t slots = (size_t)(P.npart / 32 + P.ncols + 1);
+        P.o_cmap = sizeof(unsigned long long) * (size_t)nb;
+        P.o_ccount = (P.o_cmap + sizeof(int2) * slots + 15) & ~(size_t)15;
+        P.o_segflag = P.o_ccount + sizeof(int) * (size_t)P.ncells;
+        P.cellz_bytes = P.o_segflag + sizeof(int) * (size_t)nseg;
+        JT_TRY(B->cellz.ensure(P.cellz_bytes, &grew));
     }
     JT_TRY(B->pmacc.ensure((size_t)(P.screened ? 2 : 1) * B->ngrid * std::max<int64_t>(P.npart, 1), &grew));
 
@@ -781,6 +798,27 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
     return JT_OK;
 }
 
+jt_cell_bufs cell_bufs(jt_batch* B, const Plan& P)
+{
+    jt_cell_bufs cb;
+    unsigned char* z = B->cellz.p;
+    cb.zero = z;
+    cb.zero_bytes = P.cellz_bytes;
+    cb.reach = (unsigned long long*)z;
+    cb.cmap = (int2*)(z + P.o_cmap);
+    cb.ccount = (int*)(z + P.o_ccount);
+    cb.segflag = (int*)(z + P.o_segflag);
+    cb.cstart = B->cstart.p;
+    cb.bsum = B->cbsum.p;
+    cb.ccell = B->ccell.p;
+    cb.cslot = B->cslot.p;
+    cb.cpos = B->cpos.p;
+    cb.cid = B->cid.p;
+    cb.tflag = B->tflag.p;
+    cb.dense = B->cdense.p;
+    return cb;
+}
+
 // The cell walk's cost depends on how the columns cut the particle
 // distribution (a lattice whose points fall into the columns evenly gives
 // compact full batches), which no model of the mean count predicts: the first
@@ -813,9 +851,8 @@ int tune_cells(jt_batch* B, Plan& P, int nseg, int parts, const float4* pmacc, b
     cudaStream_t st = B->st;
     const int nmax = d.nb, nmin = std::max(3, (int)std::ceil(0.7 * nmax)), dn = std::max(1, nmax / 24);
     const double rcut = jt_short_cut(bs->cfg);
-    jt_cell_bufs cb = {B->ccount.p, B->cstart.p, B->cbsum.p, B->ccell.p, B->cslot.p, B->cpos.p, B->cid.p, B->tflag.p,
-                       B->cdense.p, B->creach.p, B->cmap.p, B->csegflag.p};
-    const cudaEvent_t e0 = B->ev[8], e1 = B->ev[9];   // the pass's own events around the cell walk
+    jt_cell_bufs cb = cell_bufs(B, P);
+    const cudaEvent_t e0 = B->evs[B->evi].e[8], e1 = B->evs[B->evi].e[9];   // the pass's own events around the cell walk
     auto set_nb = [&](int nb) -> int {
         box_cells(d, bs->n[0] + bs->n[1], nb, bs->cfg, rcut);
         P.ncols = (int64_t)nb * nb;
@@ -836,9 +873,9 @@ int tune_cells(jt_batch* B, Plan& P, int nseg, int parts, const float4* pmacc, b
         for (int rep = 0; rep < 2 && r == JT_OK; rep++) {
             r = jt_b_cells(P.d_post, P.d_bx, P.d_pp, nseg, P.npart, 1, P.ncells, P.npart / 32 + P.ncols, cb,
                            B->ngrid, parts, 0.0f, nullptr, B->d_err, st, e0, e1, false, pmacc, false);
-            if (r == JT_OK && (cudaMemcpyAsync(flag, B->csegflag.p, sizeof(int) * (size_t)nseg,
+            if (r == JT_OK && (cudaMemcpyAsync(flag, cb.segflag, sizeof(int) * (size_t)nseg,
                                                cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-                               cudaMemcpyAsync(&reach, B->creach.p, sizeof(reach), cudaMemcpyDeviceToHost, st) !=
+                               cudaMemcpyAsync(&reach, cb.reach, sizeof(reach), cudaMemcpyDeviceToHost, st) !=
                                    cudaSuccess ||
                                cudaStreamSynchronize(st) != cudaSuccess))
                 r = JT_ECUDA;
@@ -879,17 +916,17 @@ int force_pass(jt_batch* B, Plan& P, int parts, float kick_frac)
 {
     cudaStream_t st = B->st;
     const int nseg = (int)P.pre.size(), nbox = (int)P.bx.size();
-    cudaEventRecord(B->ev[0], st);
-    JT_CU(cudaMemsetAsync(B->hist.p, 0, sizeof(uint32_t) * (size_t)nseg * 4 * 256, st));
-    JT_CU(cudaMemsetAsync(B->status.p, 0, sizeof(uint32_t) * (size_t)P.nsorttiles * 4 * 256, st));
-    JT_CU(cudaMemsetAsync(B->tickets.p, 0, sizeof(uint32_t) * 4, st));
-    JT_TRY(jt_b_sort_reorder(P.d_pre, P.d_bx, nseg, P.d_pp, P.npart, P.d_tp, P.nsorttiles, B->tickets.p,
+    const cudaEvent_t* ev = B->evs[B->evi].e;
+    cudaEventRecord(ev[0], st);
+    JT_CU(cudaMemsetAsync(B->sortz.p, 0,
+                          sizeof(uint32_t) * (kTickets + ((size_t)nseg + (size_t)P.nsorttiles) * 4 * 256), st));
+    JT_TRY(jt_b_sort_reorder(P.d_pre, P.d_bx, nseg, P.d_pp, P.npart, P.d_tp, P.nsorttiles, B->sortz.p,
                              B->d_err, st));
-    cudaEventRecord(B->ev[1], st);
+    cudaEventRecord(ev[1], st);
     // with the cell walk the trees are built after it, for the segments whose
     // particles it flagged (none for uniform data)
     if (!P.cells) jt_b_build_trees(P.d_post, P.d_bx, nseg, P.d_ip, P.ninternal, P.d_pp, P.npart, st);
-    cudaEventRecord(B->ev[2], st);
+    cudaEventRecord(ev[2], st);
     for (auto& kv : P.nslots) {
         const int64_t M = kv.first, G = M * M * M;
         int left = kv.second;
@@ -904,22 +941,22 @@ int force_pass(jt_batch* B, Plan& P, int parts, float kick_frac)
     const int tile = P.minT == P.maxT && (P.maxT == 16 || P.maxT == 8) ? P.maxT : 0;
     const int nsrc = P.screened ? 2 : 1;   // the unsigned source of screened boxes
     JT_TRY(jt_b_deposit(P.d_post, P.d_bx, P.d_ptp, nbox, P.npmtiles, B->order, B->ngrid, P.maxT, st, nsrc, tile));
-    cudaEventRecord(B->ev[3], st);
+    cudaEventRecord(ev[3], st);
     for (auto& kv : P.nslots) {
         Bucket& K = B->buckets[kv.first];
         JT_TRY(exec_r2c(K, kv.second, B->ngrid));
     }
-    cudaEventRecord(B->ev[4], st);
+    cudaEventRecord(ev[4], st);
     jt_b_kspace(P.d_bx, P.d_kp, nbox, P.nmodes, B->ngrid == 2, B->k_min, st);
     JT_TRY(jt_b_zfft_kspace(P.d_bx, P.d_zp, nbox, P.nztiles, B->ngrid == 2, B->k_min, 0, P.zsizes, st));
     if (P.screened)
         JT_TRY(jt_b_zfft_kspace(P.d_bx, P.d_zp, nbox, P.nztiles, B->ngrid == 2, B->k_min, 1, P.zsizes, st));
-    cudaEventRecord(B->ev[5], st);
+    cudaEventRecord(ev[5], st);
     for (auto& kv : P.nslots) {
         Bucket& K = B->buckets[kv.first];
         JT_TRY(exec_c2r(K, kv.second, B->ngrid));
     }
-    cudaEventRecord(B->ev[6], st);
+    cudaEventRecord(ev[6], st);
     // PM interpolation of every particle from shared-memory tiles
     const float4* pmacc = nullptr;
     if ((parts & JT_PART_PM) && P.npart > 0) {
@@ -928,7 +965,7 @@ int force_pass(jt_batch* B, Plan& P, int parts, float kick_frac)
         pmacc = B->pmacc.p;
         B->tm.launches += 1;
     }
-    cudaEventRecord(B->ev[10], st);
+    cudaEventRecord(ev[10], st);
     jt_tree_dev pool = {};
     pool.child = B->child.p;
     pool.range = B->range.p;
@@ -941,28 +978,29 @@ int force_pass(jt_batch* B, Plan& P, int parts, float kick_frac)
     pool.quad1 = B->quad1.p;
     pool.m30 = B->m30.p;
     const unsigned char* tflag = nullptr;
+    const int* segflag = nullptr;
     if (!P.cells) {
-        cudaEventRecord(B->ev[8], st);
-        cudaEventRecord(B->ev[9], st);
+        cudaEventRecord(ev[8], st);
+        cudaEventRecord(ev[9], st);
     } else {
         bool done = false;
         if (kick_frac == 0.0f && nbox == 1 && P.ncells > 0 && (parts & JT_PART_SHORT))
             JT_TRY(tune_cells(B, P, nseg, parts, pmacc, &done));
-        jt_cell_bufs cb = {B->ccount.p, B->cstart.p, B->cbsum.p, B->ccell.p, B->cslot.p, B->cpos.p, B->cid.p,
-                           B->tflag.p, B->cdense.p, B->creach.p, B->cmap.p, B->csegflag.p};
+        const jt_cell_bufs cb = cell_bufs(B, P);
         if (!done)
             JT_TRY(jt_b_cells(P.d_post, P.d_bx, P.d_pp, nseg, P.npart, nbox, P.ncells,
                               P.ncells > 0 ? P.npart / 32 + P.ncols : 0, cb, B->ngrid, parts, kick_frac,
-                              B->d_stats, B->d_err, st, B->ev[8], B->ev[9], P.screened, pmacc, B->counters));
+                              B->d_stats, B->d_err, st, ev[8], ev[9], P.screened, pmacc, B->counters));
         tflag = B->tflag.p;
-        jt_b_build_trees(P.d_post, P.d_bx, nseg, P.d_ip, P.ninternal, P.d_pp, P.npart, st, B->csegflag.p);
+        jt_b_build_trees(P.d_post, P.d_bx, nseg, P.d_ip, P.ninternal, P.d_pp, P.npart, st, cb.segflag);
+        segflag = cb.segflag;
         B->tm.launches += P.npart > 0 ? (P.ncells > 0 ? 6 : 1) : 0;
     }
     JT_TRY(jt_b_walk(P.d_post, P.d_bx, P.d_gp, nseg, P.ngroups, pool, B->ngrid, parts,
                      kick_frac, B->d_stats, B->d_err, st, P.d_pp, tflag, P.screened,
-                     tflag ? B->csegflag.p : nullptr, pmacc, P.npart));
-    cudaEventRecord(B->ev[7], st);
-    B->pending = true;
+                     segflag, pmacc, P.npart));
+    cudaEventRecord(ev[7], st);
+    B->evs[B->evi].pending = true;
     B->tm.launches += (P.npart > 0 ? 8 : 0) + (P.ninternal > 0 ? 1 : 0) + (P.npart > 0 ? 1 : 0) +
                       (P.npmtiles > 0 ? 2 : 0) + (P.nmodes > 0 ? 1 : 0) +
                       (P.nztiles > 0 ? (P.screened ? 2 : 1) * ((P.zsizes & 1) + ((P.zsizes >> 1) & 1)) : 0) +
@@ -981,39 +1019,48 @@ int force_pass(jt_batch* B, Plan& P, int parts, float kick_frac)
     return cudaGetLastError() == cudaSuccess ? JT_OK : JT_ECUDA;
 }
 
+// Add a finished pass's stage times to the call's timings.
+void harvest(jt_batch* B, jt_batch::Events& E)
+{
+    if (!E.pending) return;
+    const cudaEvent_t* ev = E.e;
+    B->tm.sort_ms += elapsed(ev[0], ev[1]);
+    B->tm.tree_ms += elapsed(ev[1], ev[2]);
+    B->tm.deposit_ms += elapsed(ev[2], ev[3]);
+    B->tm.fft_ms += elapsed(ev[3], ev[6]);
+    B->tm.kspace_ms += elapsed(ev[4], ev[5]);
+    B->tm.walk_ms += elapsed(ev[6], ev[7]);
+    B->tm.cellwalk_ms += elapsed(ev[8], ev[9]);
+    B->tm.interp_ms += elapsed(ev[6], ev[10]);
+    if (E.kicked) B->tm.kick_drift_ms += elapsed(ev[11], ev[12]);
+    E.pending = E.kicked = false;
+}
+
 int finish(jt_batch* B)
 {
-    unsigned e = 0;
-    unsigned long long v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    JT_CU(cudaMemcpyAsync(&e, B->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, B->st));
-    JT_CU(cudaMemcpyAsync(v, B->d_stats, sizeof(v), cudaMemcpyDeviceToHost, B->st));
+    unsigned long long* v = B->h_stats;
+    JT_CU(cudaMemcpyAsync(v, B->d_stats, 9 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, B->st));
     JT_CU(cudaStreamSynchronize(B->st));
+    const unsigned e = (unsigned)v[8];
+    unsigned long long d[8];
+    for (int i = 0; i < 8; i++) {
+        d[i] = v[i] - B->seen[i];
+        B->seen[i] = v[i];
+    }
     if (e) {
         for (jt_box_state* b : B->boxes)
             if (b) b->acc_valid = false;
         cudaMemsetAsync(B->d_err, 0, sizeof(unsigned), B->st);
-        cudaMemsetAsync(B->d_stats, 0, sizeof(v), B->st);
         cudaStreamSynchronize(B->st);
-        B->pending = false;
+        for (auto& E : B->evs) E.pending = E.kicked = false;
         return (e & JT_ERRBIT_LOOKBACK) ? JT_ETIMEDOUT : JT_EOVERFLOW;
     }
-    if (B->pending) {
-        B->tm.sort_ms += elapsed(B->ev[0], B->ev[1]);
-        B->tm.tree_ms += elapsed(B->ev[1], B->ev[2]);
-        B->tm.deposit_ms += elapsed(B->ev[2], B->ev[3]);
-        B->tm.fft_ms += elapsed(B->ev[3], B->ev[6]);
-        B->tm.kspace_ms += elapsed(B->ev[4], B->ev[5]);
-        B->tm.walk_ms += elapsed(B->ev[6], B->ev[7]);
-        B->tm.cellwalk_ms += elapsed(B->ev[8], B->ev[9]);
-        B->tm.interp_ms += elapsed(B->ev[6], B->ev[10]);
-        B->pending = false;
-    }
-    B->tm.pair_interactions += (int64_t)v[0];
-    B->tm.node_interactions += (int64_t)v[1];
-    B->tm.candidates += (int64_t)v[2];
-    B->tm.interactions += (int64_t)(v[0] + v[1]);
-    for (int i = 0; i < 4; i++) B->phase[i] += (int64_t)v[3 + i];
-    JT_CU(cudaMemsetAsync(B->d_stats, 0, sizeof(v), B->st));
+    for (auto& E : B->evs) harvest(B, E);
+    B->tm.pair_interactions += (int64_t)d[0];
+    B->tm.node_interactions += (int64_t)d[1];
+    B->tm.candidates += (int64_t)d[2];
+    B->tm.interactions += (int64_t)(d[0] + d[1]);
+    for (int i = 0; i < 4; i++) B->phase[i] += (int64_t)d[3 + i];
     return JT_OK;
 }
 
@@ -1165,7 +1212,7 @@ int capture_graphs(jt_batch* B, const std::vector<int>& v, const jt_box_step* st
     }
     const int64_t per_pass = B->tm.launches - saved.launches;
     B->tm = saved;
-    B->pending = false;
+    for (auto& E : B->evs) E.pending = E.kicked = false;   // captured, not recorded
     cudaGetLastError();
     // nothing ran during the captures: if they left the host pointers
     // swapped an odd number of times, swap them back
@@ -1355,8 +1402,8 @@ int jtb_step_host(jt_batch* B, int box_id, float* const pos[2], float* const vel
     }
     cudaStream_t st = B->st;
     B->tm = jt_timings{};
-    cudaEvent_t t0, t1, k0, k1;
-    cudaEventCreate(&t0); cudaEventCreate(&t1); cudaEventCreate(&k0); cudaEventCreate(&k1);
+    const cudaEvent_t t0 = B->ev_call[0], t1 = B->ev_call[1];
+    jt_batch::Events& E = B->evs[B->evi];
     cudaEventRecord(t0, st);
     float* io[2] = {B->io.p, B->io.p + 9 * (size_t)b->n[0]};
     int r = JT_OK;
@@ -1380,11 +1427,11 @@ int jtb_step_host(jt_batch* B, int box_id, float* const pos[2], float* const vel
     const std::vector<int> v(1, box_id);
     Plan& P = B->plan;
     if (r == JT_OK) r = build_plan(B, v, &step, P);
-    double kd = 0.0;
     if (r == JT_OK) {
-        cudaEventRecord(k0, st);
+        cudaEventRecord(E.e[11], st);
         jt_b_kick_drift(P.d_pre, P.d_bx, P.d_pp, (int)P.pre.size(), P.npart, 0.5f, 1.0f, st);
-        cudaEventRecord(k1, st);
+        cudaEventRecord(E.e[12], st);
+        E.kicked = true;
         B->tm.launches += 1;
         // the positions are final: pack them into their upload slots (still
         // in the caller's order) and copy them back while the forces run
@@ -1417,7 +1464,6 @@ int jtb_step_host(jt_batch* B, int box_id, float* const pos[2], float* const vel
                 cudaMemcpyAsync(acc[s], io[s] + 6 * n, bytes, cudaMemcpyDeviceToHost, st) != cudaSuccess)
                 r = JT_ECUDA;
         }
-        kd = elapsed(k0, k1);
         if (r == JT_OK) r = finish(B);
     }
     cudaEventRecord(t1, st);
@@ -1425,11 +1471,9 @@ int jtb_step_host(jt_batch* B, int box_id, float* const pos[2], float* const vel
     if (cudaStreamSynchronize(B->io_side) != cudaSuccess && r == JT_OK) r = JT_ECUDA;
     if (r == JT_OK) {
         B->tm.total_ms = elapsed(t0, t1);
-        B->tm.kick_drift_ms = kd;
     } else {
         b->acc_valid = false;
     }
-    cudaEventDestroy(t0); cudaEventDestroy(t1); cudaEventDestroy(k0); cudaEventDestroy(k1);
     return r;
 }
 
@@ -1461,15 +1505,17 @@ int jt_batch_create(jt_batch** out)
     cudaMemPoolSetAttribute(B->actx.pool, cudaMemPoolAttrReleaseThreshold, &keep);
     B->actx.st = B->st;
     if (const char* e = getenv("JT_COUNTERS")) B->counters = atoi(e) != 0;
-    for (auto& e : B->ev) cudaEventCreate(&e);
+    for (auto& E : B->evs)
+        for (auto& e : E.e) cudaEventCreate(&e);
+    for (auto& e : B->ev_call) cudaEventCreate(&e);
     cudaEventCreateWithFlags(&B->desc_done, cudaEventDisableTiming);
-    if (cudaMalloc(&B->d_err, sizeof(unsigned)) != cudaSuccess ||
-        cudaMalloc(&B->d_stats, 8 * sizeof(unsigned long long)) != cudaSuccess) {
+    const size_t words = 9 * sizeof(unsigned long long);
+    if (cudaMalloc(&B->d_stats, words) != cudaSuccess || cudaMallocHost((void**)&B->h_stats, words) != cudaSuccess) {
         jt_batch_destroy(B);
         return JT_ENOMEM;
     }
-    cudaMemset(B->d_err, 0, sizeof(unsigned));
-    cudaMemset(B->d_stats, 0, 8 * sizeof(unsigned long long));
+    B->d_err = (unsigned*)(B->d_stats + 8);
+    cudaMemset(B->d_stats, 0, words);
     *out = B;
     return JT_OK;
 }
@@ -1484,11 +1530,11 @@ void jt_batch_destroy(jt_batch* B)
         if (b) { box_release(b); delete b; }
     B->child.release(); B->range.release(); B->parent.release(); B->flag.release();
     B->com.release(); B->bmin.release(); B->bmax.release(); B->quad0.release(); B->quad1.release();
-    B->ccount.release(); B->cstart.release(); B->cbsum.release(); B->ccell.release(); B->cslot.release();
-    B->csegflag.release();
-    B->cpos.release(); B->cid.release(); B->cmap.release(); B->cdense.release(); B->creach.release(); B->tflag.release(); B->pmacc.release();
+    B->cstart.release(); B->cbsum.release(); B->ccell.release(); B->cslot.release();
+    B->cellz.release();
+    B->cpos.release(); B->cid.release(); B->cdense.release(); B->tflag.release(); B->pmacc.release();
     B->m30.release(); B->vals.release(); B->vals_alt.release(); B->keys_alt.release();
-    B->hist.release(); B->status.release(); B->tickets.release(); B->desc.release();
+    B->sortz.release(); B->desc.release();
     drop_graphs(B);
     B->gdesc.release();
     for (auto& kv : B->buckets) kv.second.release();
@@ -1501,9 +1547,12 @@ void jt_batch_destroy(jt_batch* B)
     }
     if (B->io_ev) cudaEventDestroy(B->io_ev);
     if (B->hdesc) cudaFreeHost(B->hdesc);
-    if (B->d_err) cudaFree(B->d_err);
     if (B->d_stats) cudaFree(B->d_stats);
-    for (auto& e : B->ev)
+    if (B->h_stats) cudaFreeHost(B->h_stats);
+    for (auto& E : B->evs)
+        for (auto& e : E.e)
+            if (e) cudaEventDestroy(e);
+    for (auto& e : B->ev_call)
         if (e) cudaEventDestroy(e);
     if (B->desc_done) cudaEventDestroy(B->desc_done);
     if (B->st) cudaStreamSynchronize(B->st);
@@ -1629,17 +1678,13 @@ int jt_batch_forces(jt_batch* B, const int* ids, int n_ids, int part)
     if (!B || part < 1 || part > 3) return JT_EINVAL;
     AllocScope scope(&B->actx);
     B->tm = jt_timings{};
-    cudaEvent_t t0, t1;
-    cudaEventCreate(&t0);
-    cudaEventCreate(&t1);
+    const cudaEvent_t t0 = B->ev_call[0], t1 = B->ev_call[1];
     cudaEventRecord(t0, B->st);
     int r = jtb_force_pass(B, ids, n_ids, part, 0.0f, nullptr);
     cudaEventRecord(t1, B->st);
     int e = finish(B);
     if (r == JT_OK) r = e;
     if (r == JT_OK) B->tm.total_ms = elapsed(t0, t1);
-    cudaEventDestroy(t0);
-    cudaEventDestroy(t1);
     return r;
 }
 
@@ -1660,8 +1705,7 @@ int jt_batch_step(jt_batch* B, const int* ids, int n_ids, const jt_step_args* ar
     }
     if (nsteps == 0) return JT_OK;
     B->tm = jt_timings{};
-    cudaEvent_t t0, t1, k0, k1;
-    cudaEventCreate(&t0); cudaEventCreate(&t1); cudaEventCreate(&k0); cudaEventCreate(&k1);
+    const cudaEvent_t t0 = B->ev_call[0], t1 = B->ev_call[1];
     cudaEventRecord(t0, B->st);
     int r = JT_OK;
     // the opening half kick needs forces at the current positions: compute
@@ -1682,7 +1726,6 @@ int jt_batch_step(jt_batch* B, const int* ids, int n_ids, const jt_step_args* ar
         r = jtb_force_pass(B, need.data(), (int)need.size(), JT_PART_ALL, 0.0f, need_steps.data());
         open_pending = r == JT_OK;
     }
-    double kd = 0.0;
     if (open_pending && B->use_graphs) {
         r = finish(B);
         open_pending = false;
@@ -1718,26 +1761,35 @@ int jt_batch_step(jt_batch* B, const int* ids, int n_ids, const jt_step_args* ar
         const int rf = finish(B);
         if (r == JT_OK) r = rf;
     }
+    // The steps queue up: the host adds a step's times while the next one runs,
+    // and reads the error word and the counters after the last.
     for (int k = 0; k < nsteps && r == JT_OK; k++) {
-        cudaEventRecord(k0, B->st);
+        jt_batch::Events& E = B->evs[B->evi];
+        cudaEventRecord(E.e[11], B->st);
         if (k == 0) jt_b_kick_drift(P.d_pre, P.d_bx, P.d_pp, (int)P.pre.size(), P.npart, 0.5f, 1.0f, B->st);
         else jt_b_drift(P.d_pre, P.d_bx, P.d_pp, (int)P.pre.size(), P.npart, 1.0f, B->st);
         B->tm.launches += 1;
-        cudaEventRecord(k1, B->st);
+        cudaEventRecord(E.e[12], B->st);
+        E.kicked = true;
         // closing half kick, merged with the next step's opening half kick
         r = force_pass(B, P, JT_PART_ALL, k + 1 < nsteps ? 1.0f : 0.5f);
         if (r != JT_OK) break;
-        r = finish(B);
-        if (r != JT_OK) break;
-        kd += elapsed(k0, k1);
+        B->evi ^= 1;
+        jt_batch::Events& before = B->evs[B->evi];   // the step before this one
+        if (before.pending) {
+            if (cudaEventSynchronize(before.e[7]) != cudaSuccess) r = JT_ECUDA;
+            else harvest(B, before);
+        }
+    }
+    if (nsteps > 0) {
+        const int rf = finish(B);   // on an error too: nothing of the call is left running
+        if (r == JT_OK) r = rf;
     }
     cudaEventRecord(t1, B->st);
     if (cudaStreamSynchronize(B->st) != cudaSuccess && r == JT_OK) r = JT_ECUDA;
     if (r == JT_OK) {
         B->tm.total_ms = elapsed(t0, t1);
-        B->tm.kick_drift_ms = kd;
     }
-    cudaEventDestroy(t0); cudaEventDestroy(t1); cudaEventDestroy(k0); cudaEventDestroy(k1);
     return r;
 }
 
@@ -1784,8 +1836,8 @@ int jt_batch_memory(jt_batch* B, size_t* persistent, size_t* scratch)
         if (b) p += b->bytes;
     s += B->child.bytes() + B->range.bytes() + B->parent.bytes() + B->flag.bytes() + B->com.bytes() +
          B->bmin.bytes() + B->bmax.bytes() + B->quad0.bytes() + B->quad1.bytes() + B->m30.bytes() +
-         B->vals.bytes() + B->vals_alt.bytes() + B->keys_alt.bytes() + B->hist.bytes() + B->status.bytes() +
-         B->tickets.bytes() + B->desc.bytes() + B->fftws.bytes() + B->gdesc.bytes() + B->stage.bytes();
+         B->vals.bytes() + B->vals_alt.bytes() + B->keys_alt.bytes() + B->sortz.bytes() +
+         B->desc.bytes() + B->fftws.bytes() + B->gdesc.bytes() + B->stage.bytes();
     for (auto& kv : B->buckets) s += (size_t)kv.second.cap * grid_bytes(kv.first, B->ngrid);
     if (persistent) *persistent = p;
     if (scratch) *scratch = s;
@@ -1839,11 +1891,11 @@ int jt_batch_trim(jt_batch* B)
     drop_graphs(B);
     B->child.release(); B->range.release(); B->parent.release(); B->flag.release();
     B->com.release(); B->bmin.release(); B->bmax.release(); B->quad0.release(); B->quad1.release();
-    B->ccount.release(); B->cstart.release(); B->cbsum.release(); B->ccell.release(); B->cslot.release();
-    B->csegflag.release();
-    B->cpos.release(); B->cid.release(); B->cmap.release(); B->cdense.release(); B->creach.release(); B->tflag.release(); B->pmacc.release();
+    B->cstart.release(); B->cbsum.release(); B->ccell.release(); B->cslot.release();
+    B->cellz.release();
+    B->cpos.release(); B->cid.release(); B->cdense.release(); B->tflag.release(); B->pmacc.release();
     B->m30.release(); B->vals.release(); B->vals_alt.release(); B->keys_alt.release();
-    B->hist.release(); B->status.release(); B->tickets.release();
+    B->sortz.release();
     for (auto& kv : B->buckets) kv.second.release();
     B->buckets.clear();
     B->fftws.release();

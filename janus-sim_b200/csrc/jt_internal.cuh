@@ -360,7 +360,10 @@ struct jt_cell_bufs {
     float4* cpos; int2* cid; unsigned char* tflag;
     unsigned char* dense;         // per block of 8 bins: above the tree walk's density
     unsigned long long* reach;    // per box: sum over its particles of the particles in reach
-    int2* cmap;                   // batch slot -> (box, column of the box), -1: none
+    int2* cmap;                   // batch slot -> (box + 1, column of the box), 0: none
+    // ccount, reach, cmap and segflag lie in one array, cleared by one memset
+    void* zero;
+    size_t zero_bytes;
     int* segflag;                 // per segment: some particle is flagged (its tree is built)
 };
 int jt_b_cells(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t* d_pprefix, int nseg,

@@ -1341,7 +1341,7 @@ __global__ void k_cell_scatter(CellArgs A, int64_t npart)
     // least ceil(count / 32) further, so no prefix sum of batch counts is needed
     const int col = (int)((key - B.cbase) / B.nbx);
     const int t0 = A.cb.cstart[B.cbase + (int64_t)col * B.nbx];
-    if (((dst - t0) & 31) == 0) A.cb.cmap[(t0 >> 5) + B.colbase + col + ((dst - t0) >> 5)] = make_int2(SG.box, col);
+    if (((dst - t0) & 31) == 0) A.cb.cmap[(t0 >> 5) + B.colbase + col + ((dst - t0) >> 5)] = make_int2(SG.box + 1, col);
 }
 
 constexpr int kCellRanges = 75;   // 25 columns, each with up to 3 images along x
@@ -1501,8 +1501,8 @@ __global__ void __launch_bounds__(kWarps * 32, kCellMinBlocks) k_walk_cell(CellA
     const int64_t slot = SPLIT > 1 ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * kWarps + wib;
     if (slot >= nslots) return;   // whole warp; with SPLIT the whole block (as the returns below)
     const int2 where = A.cb.cmap[slot];
-    if (where.x < 0) return;      // no batch in this slot
-    const jt_box_dev& B = A.boxes[where.x];
+    if (where.x == 0) return;     // no batch in this slot
+    const jt_box_dev& B = A.boxes[where.x - 1];
     const int nb = B.nb, nbx = B.nbx, col = where.y;
     const int* __restrict__ cstart = A.cb.cstart + B.cbase;
     const int tc = cstart[(int64_t)col * nbx], t1 = cstart[(int64_t)(col + 1) * nbx];
@@ -1570,7 +1570,7 @@ __global__ void __launch_bounds__(kWarps * 32, kCellMinBlocks) k_walk_cell(CellA
         }
         __syncwarp();
         if ((A.parts & 2) && nr > 0) {
-            const bool raw = (float)A.cb.reach[where.x] > B.reach_raw;
+            const bool raw = (float)A.cb.reach[where.x - 1] > B.reach_raw;
             const float ps = raw ? 1.0f : cc;   // what positions are scaled by
             const float ye = fmaxf(B.eps2 * c2, 2.3283064365386963e-10f);
             const float2* __restrict__ yt = (SCR && B.ytab) ? B.ytab : g_ltab;
@@ -1743,13 +1743,7 @@ int jt_b_cells(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_
     A.pmacc = pmacc;
     A.npart = npart;
     const unsigned gp = (unsigned)((npart + 255) / 256);
-    if (ncells > 0 && cudaMemsetAsync(cb.ccount, 0, sizeof(int) * (size_t)ncells, st) != cudaSuccess)
-        return JT_ECUDA;
-    if (nslots > 0 && cudaMemsetAsync(cb.cmap, 0xff, sizeof(int2) * (size_t)nslots, st) != cudaSuccess)
-        return JT_ECUDA;
-    if (ncells > 0 && cudaMemsetAsync(cb.reach, 0, sizeof(unsigned long long) * (size_t)nbox, st) != cudaSuccess)
-        return JT_ECUDA;
-    if (cudaMemsetAsync(cb.segflag, 0, sizeof(int) * (size_t)nseg, st) != cudaSuccess) return JT_ECUDA;
+    if (cudaMemsetAsync(cb.zero, 0, cb.zero_bytes, st) != cudaSuccess) return JT_ECUDA;
     k_cell_key<<<gp, 256, 0, st>>>(A, npart);
     if (ncells == 0) cudaEventRecord(ev_walk1, st);
     if (ncells > 0) {
