@@ -222,9 +222,10 @@ def run_clustered(J, ics, steps, warmup, H, dt, cut_tail_ppm=0, theta=0.5):
     (scale radii log-uniform 0.05-1 Mpc, species alternating by sphere) + 20 %
     uniform background, L = 100 Mpc, PM 256^3, theta 0.5, mu 19, r_s = 1.25
     cells, cut 4.5 r_s (or widened by cut_tail_ppm), softening spacing/30.
-    Most cells are too crowded for the cell walk, so the LBVH build and the
-    Barnes-Hut group walk (multipoles) do the near field.  Device time of K
-    KDK steps after W warm-up steps; the tree walk's FP32 roofline beside it."""
+    Its clumps are below the density where the tree walk's multipoles pay, so
+    the cell walk does the near field (the Barnes-Hut group walk takes denser
+    ones).  Device time of K KDK steps after W warm-up steps; the walk's FP32
+    roofline beside it."""
     n_side, L, M = 128, 100.0, 256
     n = n_side ** 3
     r_s = 1.25 * L / M
@@ -503,7 +504,7 @@ def run_serving(J, ics, n_small, n_big, steps, rates, H, dt, budget_gb=150.0):
         for cfg, st, _ in sel:
             s = J.Solver(cfg)
             s.set_state(*st)
-            s.accel()   # plans and the walk autotuner outside the timed region
+            s.accel()   # plans and the column-count timing outside the timed region
             torch.cuda.synchronize()
             t0 = time.perf_counter()
             s.set_state(*st)

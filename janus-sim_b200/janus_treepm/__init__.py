@@ -620,7 +620,7 @@ class Solver:
 
 
 def walk_tuning():
-    """The walk launch shapes the autotuner picked so far (text)."""
+    """The near-field columns per axis timed for each large box so far (text)."""
     buf = C.create_string_buffer(4096)
     _check(library().jt_walk_tuning(buf, 4096), "jt_walk_tuning")
     return buf.value.decode()
