@@ -6,7 +6,7 @@
 // this kernel transforms each (kx, ky) column along z, forms the force
 // spectra of the column (the k-space step of k_b_kspace: interlaced grids
 // combined, Green's function with the assignment deconvolution, -i k_c), and
-// transforms each of them back along z; cuFFT's 2D C2R per plane finishes the
+// transforms them back along z (x and y share a transform); cuFFT's 2D C2R per plane finishes the
 // inverse.  Against three cuFFT passes per 3D transform plus a separate
 // k-space kernel, the z passes of the 2 forward and 6 inverse transforms and
 // the k-space traffic become one read of the two spectra and one write of
