@@ -1022,7 +1022,10 @@ int force_pass(jt_batch* B, Plan& P, int parts, float kick_frac)
 // Add a finished pass's stage times to the call's timings.
 void harvest(jt_batch* B, jt_batch::Events& E)
 {
-    if (!E.pending) return;
+    if (!E.pending) {
+        E.kicked = false;   // its pass was not issued
+        return;
+    }
     const cudaEvent_t* ev = E.e;
     B->tm.sort_ms += elapsed(ev[0], ev[1]);
     B->tm.tree_ms += elapsed(ev[1], ev[2]);
