@@ -174,7 +174,8 @@ int  jt_accel_part(jt_handle* h, int part, float* acc_p, float* acc_m, int mem);
 /* Advance nsteps steps of length dt.  Kick: v += (a - H v dtau_per_dt) dt,
  * the reference's kick_f32 (:50-64) with hubble = H; drift x += v dt with
  * one periodic wrap (:33-48).  Replaces step_treepm_gpu(dt, r_cut, hubble,
- * dtau_per_dt) (:4486-4649); r_cut comes from the config. */
+ * dtau_per_dt) (:4486-4649); r_cut comes from the config.  After a device
+ * error in KDK mode the state is as jt_batch_step leaves it. */
 int  jt_step(jt_handle* h, double dt, double hubble, double dtau_per_dt, int nsteps);
 
 /* The accelerations a KDK step starts from, as part of the state: jt_get_accel
@@ -365,6 +366,10 @@ void jt_philox4x32_10(const unsigned ctr[4], const unsigned key[2], unsigned out
  * expected outcome); the device context stays usable.  No counterpart in the
  * reference. */
 int  jt_wait_probe(int limit, int* timed_out);
+/* Tests of the failure path, host side only: set the error word of an
+ * accurate-mode handle as a walk-stack overflow (JT_EOVERFLOW) or a sort
+ * time-out (JT_ETIMEDOUT) would; its next force or step call meets it. */
+int  jt_inject_error(jt_handle* h, int code);
 /* Library version string, e.g. "janus-treepm-b200 0.1 sm_100a". */
 const char* jt_version(void);
 
@@ -433,7 +438,11 @@ int  jt_batch_set_screening(jt_batch* b, int box_id, double lambda_0, double z);
 int  jt_batch_remove(jt_batch* b, int box_id);
 /* Accelerations of the listed boxes at their current positions (JT_PART_*). */
 int  jt_batch_forces(jt_batch* b, const int* box_ids, int n_ids, int part);
-/* nsteps KDK steps of the listed boxes, args[k] for box_ids[k]. */
+/* nsteps KDK steps of the listed boxes, args[k] for box_ids[k].  Steps queue
+ * up on the device.  A device error (JT_EOVERFLOW, JT_ETIMEDOUT) ends the call:
+ * the step that raised it and at most one more have advanced the state, whose
+ * positions and velocities are then not to be relied on (graphs, see
+ * jt_batch_set_graphs: all nsteps ran). */
 int  jt_batch_step(jt_batch* b, const int* box_ids, int n_ids,
                    const jt_step_args* args, int nsteps);
 /* Per-box read-back in the caller's species order (NULL pointers skipped). */

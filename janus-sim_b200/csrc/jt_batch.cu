@@ -254,7 +254,9 @@ struct jt_batch {
     // and the error word behind them, read back together
     unsigned long long* d_stats = nullptr;
     unsigned* d_err = nullptr;
-    unsigned long long* h_stats = nullptr;   // pinned
+    unsigned long long* h_stats = nullptr;   // pinned; the last word is look_for_error's
+    // reads the error word of a step that has ended while the next one runs
+    cudaStream_t err_st = nullptr;
     unsigned long long seen[8] = {};
     // two sets of a pass's stage events, used in turn, so that the steps of
     // one call queue up while the host reads the step before
@@ -1067,6 +1069,18 @@ int finish(jt_batch* B)
     return JT_OK;
 }
 
+// The error word while further work of the batch's stream is in flight (a
+// 4-byte copy on its own stream, ~10 us of the host's time): JT_OK also where
+// it is set, *set says so; finish reports and clears it.
+int look_for_error(jt_batch* B, bool* set)
+{
+    unsigned* h = (unsigned*)(B->h_stats + 9);
+    JT_CU(cudaMemcpyAsync(h, B->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, B->err_st));
+    JT_CU(cudaStreamSynchronize(B->err_st));
+    *set = *h != 0;
+    return JT_OK;
+}
+
 int valid_ids(jt_batch* B, const int* ids, int n, std::vector<int>& out)
 {
     out.clear();
@@ -1302,6 +1316,15 @@ void jtb_reset_timings(jt_batch* B)
     if (B) B->tm = jt_timings{};
 }
 
+int jtb_inject_error(jt_batch* B, int code)
+{
+    if (!B || (code != JT_EOVERFLOW && code != JT_ETIMEDOUT)) return JT_EINVAL;
+    const unsigned bits = code == JT_ETIMEDOUT ? JT_ERRBIT_LOOKBACK : JT_ERRBIT_STACK;
+    JT_CU(cudaMemcpyAsync(B->d_err, &bits, sizeof(bits), cudaMemcpyHostToDevice, B->st));
+    JT_CU(cudaStreamSynchronize(B->st));
+    return JT_OK;
+}
+
 jt_ckpt** jtb_ckpt_slot(jt_batch* B) { return &B->ckpt; }
 int64_t jtb_phase(jt_batch* B, int i) { return B && i >= 0 && i < 4 ? B->phase[i] : 0; }
 
@@ -1513,9 +1536,14 @@ int jt_batch_create(jt_batch** out)
     for (auto& e : B->ev_call) cudaEventCreate(&e);
     cudaEventCreateWithFlags(&B->desc_done, cudaEventDisableTiming);
     const size_t words = 9 * sizeof(unsigned long long);
-    if (cudaMalloc(&B->d_stats, words) != cudaSuccess || cudaMallocHost((void**)&B->h_stats, words) != cudaSuccess) {
+    if (cudaMalloc(&B->d_stats, words) != cudaSuccess ||
+        cudaMallocHost((void**)&B->h_stats, words + sizeof(unsigned long long)) != cudaSuccess) {
         jt_batch_destroy(B);
         return JT_ENOMEM;
+    }
+    if (cudaStreamCreateWithFlags(&B->err_st, cudaStreamNonBlocking) != cudaSuccess) {
+        jt_batch_destroy(B);
+        return JT_ECUDA;
     }
     B->d_err = (unsigned*)(B->d_stats + 8);
     cudaMemset(B->d_stats, 0, words);
@@ -1552,6 +1580,7 @@ void jt_batch_destroy(jt_batch* B)
     if (B->hdesc) cudaFreeHost(B->hdesc);
     if (B->d_stats) cudaFree(B->d_stats);
     if (B->h_stats) cudaFreeHost(B->h_stats);
+    if (B->err_st) cudaStreamDestroy(B->err_st);
     for (auto& E : B->evs)
         for (auto& e : E.e)
             if (e) cudaEventDestroy(e);
@@ -1764,9 +1793,11 @@ int jt_batch_step(jt_batch* B, const int* ids, int n_ids, const jt_step_args* ar
         const int rf = finish(B);
         if (r == JT_OK) r = rf;
     }
-    // The steps queue up: the host adds a step's times while the next one runs,
-    // and reads the error word and the counters after the last.
-    for (int k = 0; k < nsteps && r == JT_OK; k++) {
+    // The steps queue up: while one runs, the host adds the times of the one
+    // before and looks at its error word, so that a failed step is followed by
+    // one more at most; the counters are read after the last.
+    bool failed = false;
+    for (int k = 0; k < nsteps && r == JT_OK && !failed; k++) {
         jt_batch::Events& E = B->evs[B->evi];
         cudaEventRecord(E.e[11], B->st);
         if (k == 0) jt_b_kick_drift(P.d_pre, P.d_bx, P.d_pp, (int)P.pre.size(), P.npart, 0.5f, 1.0f, B->st);
@@ -1780,8 +1811,12 @@ int jt_batch_step(jt_batch* B, const int* ids, int n_ids, const jt_step_args* ar
         B->evi ^= 1;
         jt_batch::Events& before = B->evs[B->evi];   // the step before this one
         if (before.pending) {
-            if (cudaEventSynchronize(before.e[7]) != cudaSuccess) r = JT_ECUDA;
-            else harvest(B, before);
+            if (cudaEventSynchronize(before.e[7]) != cudaSuccess) {
+                r = JT_ECUDA;
+            } else {
+                harvest(B, before);
+                r = look_for_error(B, &failed);
+            }
         }
     }
     if (nsteps > 0) {

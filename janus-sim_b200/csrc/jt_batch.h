@@ -55,6 +55,8 @@ int jtb_force_pass(jt_batch* B, const int* ids, int n_ids, int parts, float kick
 // Synchronise, read the device error word and add the pass's stage times.
 int jtb_finish(jt_batch* B);
 void jtb_reset_timings(jt_batch* B);
+// jt_inject_error on a batch
+int jtb_inject_error(jt_batch* B, int code);
 int64_t jtb_phase(jt_batch* B, int i);
 // Set a box's accelerations (species AoS float3 in the caller's order, host
 // or device) and mark them valid for its current positions; used to restore

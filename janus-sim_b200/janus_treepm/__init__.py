@@ -45,7 +45,7 @@ EXPORTED = [
     "jt_batch_trim", "jt_batch_set_graphs", "jt_server_create", "jt_server_destroy",
     "jt_server_add_job", "jt_server_request", "jt_server_clock", "jt_server_poll", "jt_server_serve",
     "jt_server_job_state", "jt_server_get_state", "jt_server_stats", "jt_server_job_need",
-    "jt_walk_tuning", "jt_wait_probe", "jt_diagnostics", "jt_batch_diagnostics",
+    "jt_walk_tuning", "jt_wait_probe", "jt_inject_error", "jt_diagnostics", "jt_batch_diagnostics",
     "jt_snapshot_write", "jt_snapshot_read", "jt_checkpoint", "jt_set_screening",
     "jt_ics_zeldovich", "jt_set_state_zeldovich", "jt_batch_add_zeldovich", "jt_philox4x32_10",
     "jt_energy_sampled", "jt_virialize_sampled", "jt_energy_drift_pct",
@@ -301,6 +301,7 @@ def library():
     L.jt_batch_get_timings.argtypes = [H, C.POINTER(jt_timings)]
     L.jt_morton_sort_static.argtypes = [vp, C.c_size_t, C.c_double, vp, vp, vp]
     L.jt_walk_tuning.argtypes = [C.c_char_p, C.c_size_t]
+    L.jt_inject_error.argtypes = [H, C.c_int]
     L.jt_wait_probe.argtypes = [C.c_int, C.POINTER(C.c_int)]
     L.jt_diagnostics.argtypes = [H, C.c_int, C.POINTER(jt_diag)]
     L.jt_snapshot_write.argtypes = [C.c_char_p, C.POINTER(jt_snapshot_meta), C.c_double, C.c_double,

@@ -36,3 +36,28 @@ def test_probe_rejects_bad_limits():
     flag = C.c_int()
     assert J.library().jt_wait_probe(0, C.byref(flag)) == J.JT_EINVAL
     assert J.library().jt_wait_probe(1 << 25, C.byref(flag)) == J.JT_EINVAL
+
+
+@pytest.mark.parametrize("code", [J.JT_EOVERFLOW, J.JT_ETIMEDOUT])
+def test_device_error_ends_a_call_of_many_steps(code):
+    """The error word is set before the call: the step that meets it and at most
+    one more run (drifts of dt v show how many), the call reports the error, and
+    the next call works."""
+    n, dt, v = 300, 0.25, 0.125
+    rng = np.random.default_rng(2)
+    pp = rng.uniform(-16, 0, (n, 3)).astype(np.float32)
+    vp = np.full((n, 3), v, np.float32)
+    s = J.Solver(J.Config(box_L=32.0, pm_grid=32, softening=0.05, G_mass_plus=1e-12))
+    s.set_state(pp, vp, pp[:0], vp[:0])
+    s.accel()
+    assert J.library().jt_inject_error(s._h, code) == J.JT_OK
+    with pytest.raises(J.JanusError) as e:
+        s.step(dt, 0.0, 1.0, 12)
+    assert e.value.code == code
+    steps = (s.get_state()[0] - pp) / (dt * v)
+    assert 0.99 < steps.min() and steps.max() < 2.01, (steps.min(), steps.max())
+    s.step(dt, 0.0, 1.0, 3)
+    steps2 = (s.get_state()[0] - pp) / (dt * v) - steps
+    assert np.abs(steps2 - 3).max() < 0.01
+    assert J.library().jt_inject_error(s._h, J.JT_EBUSY) == J.JT_EINVAL
+    s.close()
