@@ -368,7 +368,8 @@ void jt_philox4x32_10(const unsigned ctr[4], const unsigned key[2], unsigned out
 int  jt_wait_probe(int limit, int* timed_out);
 /* Tests of the failure path, host side only: set the error word of an
  * accurate-mode handle as a walk-stack overflow (JT_EOVERFLOW) or a sort
- * time-out (JT_ETIMEDOUT) would; its next force or step call meets it. */
+ * time-out (JT_ETIMEDOUT) would, or let its next force pass fail on the host
+ * before it launches anything (JT_ECUDA); the next force or step call meets it. */
 int  jt_inject_error(jt_handle* h, int code);
 /* Library version string, e.g. "janus-treepm-b200 0.1 sm_100a". */
 const char* jt_version(void);

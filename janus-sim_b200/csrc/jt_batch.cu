@@ -270,6 +270,7 @@ struct jt_batch {
     cudaEvent_t ev_call[2] = {};        // around a call
     bool counters = false;              // the cell walk counts its pairs (jt_batch_set_counters)
     bool cell_tune = true;              // tune_cells may run (jtb_set_cell_tune)
+    bool fail_next = false;             // the next force pass fails on the host (jt_inject_error)
     jt_timings tm = {};
     int64_t phase[4] = {0, 0, 0, 0};
     Plan plan;
@@ -919,6 +920,10 @@ int force_pass(jt_batch* B, Plan& P, int parts, float kick_frac)
     cudaStream_t st = B->st;
     const int nseg = (int)P.pre.size(), nbox = (int)P.bx.size();
     const cudaEvent_t* ev = B->evs[B->evi].e;
+    if (B->fail_next) {
+        B->fail_next = false;
+        return JT_ECUDA;
+    }
     cudaEventRecord(ev[0], st);
     JT_CU(cudaMemsetAsync(B->sortz.p, 0,
                           sizeof(uint32_t) * (kTickets + ((size_t)nseg + (size_t)P.nsorttiles) * 4 * 256), st));
@@ -1318,7 +1323,11 @@ void jtb_reset_timings(jt_batch* B)
 
 int jtb_inject_error(jt_batch* B, int code)
 {
-    if (!B || (code != JT_EOVERFLOW && code != JT_ETIMEDOUT)) return JT_EINVAL;
+    if (!B || (code != JT_EOVERFLOW && code != JT_ETIMEDOUT && code != JT_ECUDA)) return JT_EINVAL;
+    if (code == JT_ECUDA) {
+        B->fail_next = true;
+        return JT_OK;
+    }
     const unsigned bits = code == JT_ETIMEDOUT ? JT_ERRBIT_LOOKBACK : JT_ERRBIT_STACK;
     JT_CU(cudaMemcpyAsync(B->d_err, &bits, sizeof(bits), cudaMemcpyHostToDevice, B->st));
     JT_CU(cudaStreamSynchronize(B->st));
@@ -1490,8 +1499,9 @@ int jtb_step_host(jt_batch* B, int box_id, float* const pos[2], float* const vel
                 cudaMemcpyAsync(acc[s], io[s] + 6 * n, bytes, cudaMemcpyDeviceToHost, st) != cudaSuccess)
                 r = JT_ECUDA;
         }
-        if (r == JT_OK) r = finish(B);
     }
+    const int rf = finish(B);   // on an error too: nothing of it is left for the next call
+    if (r == JT_OK) r = rf;
     cudaEventRecord(t1, st);
     if (cudaStreamSynchronize(st) != cudaSuccess && r == JT_OK) r = JT_ECUDA;
     if (cudaStreamSynchronize(B->io_side) != cudaSuccess && r == JT_OK) r = JT_ECUDA;

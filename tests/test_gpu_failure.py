@@ -61,3 +61,28 @@ def test_device_error_ends_a_call_of_many_steps(code):
     assert np.abs(steps2 - 3).max() < 0.01
     assert J.library().jt_inject_error(s._h, J.JT_EBUSY) == J.JT_EINVAL
     s.close()
+
+
+def test_failed_host_step_leaves_nothing_for_the_next_call():
+    """A round trip whose force pass fails on the host: its kick and drift are
+    not in the next call's timings, and the round trip works again."""
+    rng = np.random.default_rng(3)
+    pp = rng.uniform(-15, 15, (900, 3)).astype(np.float32)
+    pm = rng.uniform(-15, 15, (800, 3)).astype(np.float32)
+    s = J.Solver(J.Config(box_L=32.0, pm_grid=32, softening=0.05))
+    s.set_state(pp, None, pm, None)
+    ap, am = s.accel()
+    state = [pp.copy(), np.zeros_like(pp), ap.copy(), pm.copy(), np.zeros_like(pm), am.copy()]
+    assert J.library().jt_inject_error(s._h, J.JT_ECUDA) == J.JT_OK
+    with pytest.raises(J.JanusError) as e:
+        s.step_host(*[a.copy() for a in state], 1e-3, 0.0, 1.0)
+    assert e.value.code == J.JT_ECUDA
+    s.accel()
+    assert s.timings()["kick_drift_ms"] == 0.0
+    s.step_host(*state, 1e-3, 0.0, 1.0)
+    t = s.timings()
+    assert 0.0 < t["kick_drift_ms"] < t["total_ms"]
+    s.set_state(pp, None, pm, None)
+    s.step(1e-3, 0.0, 1.0, 1)
+    assert np.abs(s.get_state()[0] - state[0]).max() < 1e-5
+    s.close()
