@@ -251,7 +251,8 @@ struct jt_batch {
     cudaEvent_t desc_done = nullptr;    // the last upload from hdesc finished
     std::map<int, Bucket> buckets;
     // pair counters (8 words, never reset: the host keeps what it has read)
-    // and the error word behind them, read back together
+    // and the error word behind them, read back together; 8 more counters for
+    // the timing runs of tune_cells
     unsigned long long* d_stats = nullptr;
     unsigned* d_err = nullptr;
     unsigned long long* h_stats = nullptr;   // pinned; the last word is look_for_error's
@@ -836,7 +837,7 @@ std::mutex g_cell_tune_mu;
 std::string g_cell_tune_text;   // one entry per timed box (jt_cell_tuning_text)
 
 // *done: the pass's cell walk has already run (a clustered box keeps the default,
-// which the first timing run left in place).
+// which the first timing run left in place; its counters go into the call's timings).
 int tune_cells(jt_batch* B, Plan& P, int nseg, int parts, const float4* pmacc, bool* done)
 {
     jt_box_state* bs = B->boxes[P.ids[0]];
@@ -867,18 +868,22 @@ int tune_cells(jt_batch* B, Plan& P, int nseg, int parts, const float4* pmacc, b
     int r = JT_OK, best = nmax;
     bool crowded = false;
     float best_ms = 0.f;
+    unsigned long long* stats = B->d_stats + 9;   // counted as in the pass itself
+    if (cudaMemsetAsync(stats, 0, 8 * sizeof(*stats), st) != cudaSuccess) return JT_ECUDA;
     for (int nb = nmax; nb >= nmin && r == JT_OK; nb -= dn) {
         r = set_nb(nb);
         // two runs, the faster one counts (candidates a few % apart)
         float ms = 0.f;
         int flag[2] = {0, 0};
-        unsigned long long reach = 0;
+        unsigned long long reach = 0, count[3] = {0, 0, 0};
         for (int rep = 0; rep < 2 && r == JT_OK; rep++) {
             r = jt_b_cells(P.d_post, P.d_bx, P.d_pp, nseg, P.npart, 1, P.ncells, P.npart / 32 + P.ncols, cb,
-                           B->ngrid, parts, 0.0f, nullptr, B->d_err, st, e0, e1, false, pmacc, false);
+                           B->ngrid, parts, 0.0f, stats, B->d_err, st, e0, e1, false, pmacc, false);
             if (r == JT_OK && (cudaMemcpyAsync(flag, cb.segflag, sizeof(int) * (size_t)nseg,
                                                cudaMemcpyDeviceToHost, st) != cudaSuccess ||
                                cudaMemcpyAsync(&reach, cb.reach, sizeof(reach), cudaMemcpyDeviceToHost, st) !=
+                                   cudaSuccess ||
+                               cudaMemcpyAsync(count, stats, sizeof(count), cudaMemcpyDeviceToHost, st) !=
                                    cudaSuccess ||
                                cudaStreamSynchronize(st) != cudaSuccess))
                 r = JT_ECUDA;
@@ -890,7 +895,14 @@ int tune_cells(jt_batch* B, Plan& P, int nseg, int parts, const float4* pmacc, b
             if (r == JT_OK && nb == nmax) {
                 const double n = (double)(bs->n[0] + bs->n[1]);
                 crowded = flag[0] || flag[1] || (double)reach > 2.0 * n * n * uniform_reach(d);
-                if (crowded) break;
+                if (crowded) {
+                    if (!B->counters) {
+                        B->tm.pair_interactions += (int64_t)count[0];
+                        B->tm.interactions += (int64_t)count[0];
+                        B->tm.candidates += (int64_t)count[2];
+                    }
+                    break;
+                }
             }
         }
         if (r != JT_OK || crowded) break;
@@ -1545,9 +1557,9 @@ int jt_batch_create(jt_batch** out)
         for (auto& e : E.e) cudaEventCreate(&e);
     for (auto& e : B->ev_call) cudaEventCreate(&e);
     cudaEventCreateWithFlags(&B->desc_done, cudaEventDisableTiming);
-    const size_t words = 9 * sizeof(unsigned long long);
+    const size_t words = 17 * sizeof(unsigned long long);
     if (cudaMalloc(&B->d_stats, words) != cudaSuccess ||
-        cudaMallocHost((void**)&B->h_stats, words + sizeof(unsigned long long)) != cudaSuccess) {
+        cudaMallocHost((void**)&B->h_stats, 10 * sizeof(unsigned long long)) != cudaSuccess) {
         jt_batch_destroy(B);
         return JT_ENOMEM;
     }

@@ -131,3 +131,27 @@ def test_boxes_of_every_route_in_one_pass():
             if len(r):
                 rms = max(float(np.sqrt((r.astype(np.float64) ** 2).sum(1).mean())), 1e-30)
                 assert np.abs(a - r).max() <= 2e-5 * max(rms, float(np.abs(r).max()))
+
+
+def test_first_pass_of_a_large_clustered_box_counts_its_candidates():
+    """The pass that times the column counts keeps its first run in a clustered
+    box; that run's candidates are the pass's."""
+    import janus_treepm as J
+    n, L = 1 << 21, 100.0
+    cfg = _config(J, L, 256, 4.5, 0.5, 2 * n)
+    s = J.Solver(cfg)
+    rng = np.random.default_rng(4)
+    centres = (rng.random((64, 3)) - 0.5) * L
+
+    def points():
+        x = centres[rng.integers(0, 64, n)] + rng.normal(0.0, 1.5, (n, 3))
+        return (np.remainder(x + 0.5 * L, L) - 0.5 * L).clip(-0.49999 * L, 0.49999 * L).astype(np.float32)
+
+    s.set_state(points(), None, points(), None)
+    s.accel()
+    first = s.timings()["candidates"]
+    s.accel()
+    again = s.timings()["candidates"]
+    s.close()
+    # the second pass's cells hold the same particles in another order
+    assert again > 0 and abs(first - again) < 0.02 * again, (first, again)
