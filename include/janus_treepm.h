@@ -366,6 +366,21 @@ void jt_philox4x32_10(const unsigned ctr[4], const unsigned key[2], unsigned out
  * expected outcome); the device context stays usable.  No counterpart in the
  * reference. */
 int  jt_wait_probe(int limit, int* timed_out);
+/* The near-field cell list of a box in accurate mode: nb columns per axis
+ * (0: none, the tree walk takes every particle) of nbx bins along x, and the
+ * columns in reach on either side of a batch's own; the particles that a
+ * target has in reach in a uniform box.  jt_cell_layout computes these on the
+ * host (a box whose columns were timed may use fewer); jt_debug_cells gives
+ * them for a handle's last force pass, with the mean number in reach, the
+ * targets that the tree walk took, and whether the box counts as clustered
+ * (its differences are taken of unscaled positions). */
+typedef struct jt_cell_info {
+    int nb, nbx, colm, unscaled;
+    int64_t to_tree;
+    double reach, reach_uniform;
+} jt_cell_info;
+int  jt_cell_layout(const jt_config* cfg, size_t n_p, size_t n_m, jt_cell_info* out);
+int  jt_debug_cells(jt_handle* h, jt_cell_info* out);
 /* Tests of the failure path, host side only: set the error word of an
  * accurate-mode handle as a walk-stack overflow (JT_EOVERFLOW) or a sort
  * time-out (JT_ETIMEDOUT) would, or let its next force pass fail on the host

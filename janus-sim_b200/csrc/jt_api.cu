@@ -888,6 +888,12 @@ int jt_step(jt_handle* h, double dt, double hubble, double dtau_per_dt, int nste
     return r;
 }
 
+int jt_debug_cells(jt_handle* h, jt_cell_info* out)
+{
+    if (!h || !out || !h->batch) return JT_EINVAL;
+    return jtb_cell_info(h->batch, out);
+}
+
 int jt_inject_error(jt_handle* h, int code) { return h && h->batch ? jtb_inject_error(h->batch, code) : JT_EINVAL; }
 
 int jt_step_host(jt_handle* h, float* pos_p, float* vel_p, float* acc_p, float* pos_m, float* vel_m,

@@ -546,8 +546,8 @@ int cell_columns(double L, double rcut, int64_t n)
 // the share of a uniform box's particles that a block has in reach (k_cell_dense)
 double uniform_reach(const jt_box_dev& d)
 {
-    const double w = 2 * d.colm + 1, nb = d.nb;
-    return std::min(1.0, w * w * std::min(w, nb) / (nb * nb * nb));
+    const double w = std::min(2 * d.colm + 1, d.nb) / (double)d.nb;
+    return w * w * w;
 }
 
 // the cell list of a box with nb columns per axis
@@ -565,6 +565,19 @@ void box_cells(jt_box_dev& d, int64_t n, int nb, const jt_config& c, double rcut
     d.cell_dmax = (float)(JT_CELL_KMAX / (27.0 * c.r_cut * c.r_cut * c.r_cut) * bin);
     d.reach_max = (float)(JT_CELL_REACH / c.theta * (double)n);   // theta 0: no multipoles, never
     d.reach_raw = (float)(1.3 * (double)n * (double)n * uniform_reach(d));
+}
+
+// whether the box has a cell list (at least three cuts along it), and its layout
+bool box_has_cells(const jt_config& c, double rcut) { return rcut > 0.0 && c.box_L >= 3.0 * 1.0001 * rcut; }
+
+jt_cell_info cell_layout_info(const jt_box_dev& d, double n)
+{
+    jt_cell_info o = {};
+    o.nb = d.nb;
+    o.nbx = d.nbx;
+    o.colm = d.nb ? d.colm : 0;
+    o.reach_uniform = d.nb ? n * uniform_reach(d) : 0.0;
+    return o;
 }
 
 constexpr size_t kTickets = 32;   // words before the sort's counts (one ticket per pass)
@@ -690,7 +703,7 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
         // tree walk only
         d.cbase = P.ncells;
         d.colbase = P.ncols;
-        if (P.cells && rcut > 0.0 && c.box_L >= 3.0 * 1.0001 * rcut)
+        if (P.cells && box_has_cells(c, rcut))
             box_cells(d, b->n[0] + b->n[1], b->cell_nb > 0 ? b->cell_nb : cell_columns(c.box_L, rcut, b->n[0] + b->n[1]), c, rcut);
         P.ncells += (int64_t)d.nb * d.nb * d.nbx;
         P.ncols += (int64_t)d.nb * d.nb;
@@ -1114,6 +1127,25 @@ int valid_ids(jt_batch* B, const int* ids, int n, std::vector<int>& out)
 
 }  // namespace
 
+int jtb_cell_info(jt_batch* B, jt_cell_info* out)
+{
+    const Plan& P = B->plan;
+    if (P.bx.size() != 1 || !P.cells || P.npart <= 0) return JT_ESTATE;
+    const jt_box_dev& d = P.bx[0];
+    *out = cell_layout_info(d, (double)P.npart);
+    if (d.nb == 0) return JT_OK;
+    const jt_cell_bufs cb = cell_bufs(B, P);
+    unsigned long long reach = 0;
+    std::vector<unsigned char> flags((size_t)P.npart);
+    JT_CU(cudaMemcpyAsync(&reach, cb.reach, sizeof(reach), cudaMemcpyDeviceToHost, B->st));
+    JT_CU(cudaMemcpyAsync(flags.data(), cb.tflag, flags.size(), cudaMemcpyDeviceToHost, B->st));
+    JT_CU(cudaStreamSynchronize(B->st));
+    for (unsigned char f : flags) out->to_tree += f ? 1 : 0;
+    out->reach = (double)reach / (double)P.npart;
+    out->unscaled = (float)reach > d.reach_raw ? 1 : 0;
+    return JT_OK;
+}
+
 double jt_short_cut(const jt_config& c)
 {
     if (c.cut_tail_ppm <= 0 || !(c.r_s > 0.0)) return c.r_cut;
@@ -1527,6 +1559,18 @@ int jtb_step_host(jt_batch* B, int box_id, float* const pos[2], float* const vel
 
 // ---------------------------------------------------------------- C ABI
 extern "C" {
+
+int jt_cell_layout(const jt_config* cfg, size_t n_p, size_t n_m, jt_cell_info* out)
+{
+    if (!out || n_p + n_m == 0 || n_p >= (size_t)1 << 30 || n_m >= (size_t)1 << 30) return JT_EINVAL;
+    JT_TRY(validate_box_config(cfg));
+    const int64_t n = (int64_t)(n_p + n_m);
+    const double rcut = jt_short_cut(*cfg);
+    jt_box_dev d = {};
+    if (box_has_cells(*cfg, rcut)) box_cells(d, n, cell_columns(cfg->box_L, rcut, n), *cfg, rcut);
+    *out = cell_layout_info(d, (double)n);
+    return JT_OK;
+}
 
 int jt_batch_create(jt_batch** out)
 {

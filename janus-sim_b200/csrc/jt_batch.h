@@ -55,6 +55,8 @@ int jtb_force_pass(jt_batch* B, const int* ids, int n_ids, int parts, float kick
 // Synchronise, read the device error word and add the pass's stage times.
 int jtb_finish(jt_batch* B);
 void jtb_reset_timings(jt_batch* B);
+// jt_debug_cells of a batch whose last pass held one box
+int jtb_cell_info(jt_batch* B, jt_cell_info* out);
 // jt_inject_error on a batch
 int jtb_inject_error(jt_batch* B, int code);
 int64_t jtb_phase(jt_batch* B, int i);

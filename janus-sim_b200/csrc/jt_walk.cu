@@ -1290,19 +1290,19 @@ __global__ void __launch_bounds__(256) k_cell_dense(const jt_box_dev* __restrict
         bool dense = false;
         if (n > 0) {
             const int kx = (int)(local % nb), cy = (int)((local / nb) % nb), cz = (int)(local / ((int64_t)nb * nb));
-            const int span = min(w, nb);   // blocks along x
+            const int span = min(w, nb);   // blocks per axis: each of a small box's once
             const int x0 = w > nb ? 0 : kx - m, x1 = x0 + span;
             int tot = 0;
-            if (lane < w * w) {
-                const int dy = lane % w - m, dz = lane / w - m;
-                const int* __restrict__ c = cstart + ((int64_t)((cz + dz + nb) % nb) * nb + (cy + dy + nb) % nb) * B.nbx;
+            if (lane < span * span) {
+                const int ny = cy - m + lane % span + nb, nz = cz - m + lane / span + nb;
+                const int* __restrict__ c = cstart + ((int64_t)(nz % nb) * nb + ny % nb) * B.nbx;
                 tot = c[8 * min(x1, nb)] - c[8 * max(x0, 0)];
                 if (x0 < 0) tot += c[8 * nb] - c[8 * (nb + x0)];
                 if (x1 > nb) tot += c[8 * (x1 - nb)] - c[0];
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-            dense = (float)tot > B.cell_dmax * (float)(8 * span * w * w);
+            dense = (float)tot > B.cell_dmax * (float)(8 * span * span * span);
             work += (unsigned long long)n * (unsigned long long)tot;
         }
         if (lane == 0) cb.dense[q] = dense ? 1 : 0;

@@ -45,7 +45,7 @@ EXPORTED = [
     "jt_batch_trim", "jt_batch_set_graphs", "jt_server_create", "jt_server_destroy",
     "jt_server_add_job", "jt_server_request", "jt_server_clock", "jt_server_poll", "jt_server_serve",
     "jt_server_job_state", "jt_server_get_state", "jt_server_stats", "jt_server_job_need",
-    "jt_walk_tuning", "jt_wait_probe", "jt_inject_error", "jt_diagnostics", "jt_batch_diagnostics",
+    "jt_walk_tuning", "jt_wait_probe", "jt_inject_error", "jt_cell_layout", "jt_debug_cells", "jt_diagnostics", "jt_batch_diagnostics",
     "jt_snapshot_write", "jt_snapshot_read", "jt_checkpoint", "jt_set_screening",
     "jt_ics_zeldovich", "jt_set_state_zeldovich", "jt_batch_add_zeldovich", "jt_philox4x32_10",
     "jt_energy_sampled", "jt_virialize_sampled", "jt_energy_drift_pct",
@@ -66,6 +66,11 @@ class JanusError(RuntimeError):
         self.code = code
         msg = _strerror(code)
         super().__init__(f"{what}: {msg} ({code})" if what else f"{msg} ({code})")
+
+
+class jt_cell_info(C.Structure):
+    _fields_ = [(k, C.c_int) for k in ("nb", "nbx", "colm", "unscaled")] + \
+               [("to_tree", C.c_int64), ("reach", C.c_double), ("reach_uniform", C.c_double)]
 
 
 class jt_config(C.Structure):
@@ -302,6 +307,8 @@ def library():
     L.jt_morton_sort_static.argtypes = [vp, C.c_size_t, C.c_double, vp, vp, vp]
     L.jt_walk_tuning.argtypes = [C.c_char_p, C.c_size_t]
     L.jt_inject_error.argtypes = [H, C.c_int]
+    L.jt_cell_layout.argtypes = [C.POINTER(jt_config), C.c_size_t, C.c_size_t, C.POINTER(jt_cell_info)]
+    L.jt_debug_cells.argtypes = [H, C.POINTER(jt_cell_info)]
     L.jt_wait_probe.argtypes = [C.c_int, C.POINTER(C.c_int)]
     L.jt_diagnostics.argtypes = [H, C.c_int, C.POINTER(jt_diag)]
     L.jt_snapshot_write.argtypes = [C.c_char_p, C.POINTER(jt_snapshot_meta), C.c_double, C.c_double,
@@ -613,6 +620,12 @@ class Solver:
         v = (C.c_int64 * 4)()
         _check(library().jt_walk_counters(self._h, v), "jt_walk_counters")
         return tuple(v)
+
+    def cells(self):
+        """The cell list and the routing of the last force pass (jt_debug_cells)."""
+        o = jt_cell_info()
+        _check(library().jt_debug_cells(self._h, C.byref(o)), "jt_debug_cells")
+        return {k: getattr(o, k) for k, _ in o._fields_}
 
     def timings(self):
         t = jt_timings()
@@ -1064,6 +1077,13 @@ class TreePMForce:
 
 def version():
     return library().jt_version().decode()
+
+
+def cell_layout(config, n_p, n_m):
+    """The near-field cell list of a box (jt_cell_info as a dict); no device work."""
+    cfg, o = config.resolved().to_c(), jt_cell_info()
+    _check(library().jt_cell_layout(C.byref(cfg), n_p, n_m, C.byref(o)), "jt_cell_layout")
+    return {k: getattr(o, k) for k, _ in o._fields_}
 
 
 def short_cut(config):

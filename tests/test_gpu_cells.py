@@ -155,3 +155,17 @@ def test_first_pass_of_a_large_clustered_box_counts_its_candidates():
     s.close()
     # the second pass's cells hold the same particles in another order
     assert again > 0 and abs(first - again) < 0.02 * again, (first, again)
+
+
+@pytest.mark.parametrize("n,nb", [(20, 1), (300, 2), (1000, 3), (2500, 4), (4100, 5)])
+def test_a_small_uniform_box_is_not_clustered(n, nb):
+    """Every column of these boxes is in reach of every other, and counts once."""
+    import janus_treepm as J
+    cfg = _config(J, 20.0, 16, 4.1, 0.5, n)
+    s = J.Solver(cfg)
+    s.set_state(_points("uniform", n // 2, 20.0, 5), None, _points("uniform", n - n // 2, 20.0, 6), None)
+    s.accel()
+    c = s.cells()
+    s.close()
+    assert c["nb"] == nb and 2 * c["colm"] + 1 >= nb
+    assert c["reach"] == c["reach_uniform"] == n and c["unscaled"] == 0 and c["to_tree"] == 0
