@@ -141,10 +141,10 @@ def test_first_pass_of_a_large_clustered_box_counts_its_candidates():
     cfg = _config(J, L, 256, 4.5, 0.5, 2 * n)
     s = J.Solver(cfg)
     rng = np.random.default_rng(4)
-    centres = (rng.random((64, 3)) - 0.5) * L
+    centres = (rng.random((512, 3)) - 0.5) * L   # not so dense that the tree walk takes them
 
     def points():
-        x = centres[rng.integers(0, 64, n)] + rng.normal(0.0, 1.5, (n, 3))
+        x = centres[rng.integers(0, 512, n)] + rng.normal(0.0, 1.0, (n, 3))
         return (np.remainder(x + 0.5 * L, L) - 0.5 * L).clip(-0.49999 * L, 0.49999 * L).astype(np.float32)
 
     s.set_state(points(), None, points(), None)
@@ -152,7 +152,9 @@ def test_first_pass_of_a_large_clustered_box_counts_its_candidates():
     first = s.timings()["candidates"]
     s.accel()
     again = s.timings()["candidates"]
+    c = s.cells()
     s.close()
+    assert c["reach"] > 2.0 * c["reach_uniform"] and c["to_tree"] == 0, c
     # the second pass's cells hold the same particles in another order
     assert again > 0 and abs(first - again) < 0.02 * again, (first, again)
 
