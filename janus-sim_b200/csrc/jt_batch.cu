@@ -550,8 +550,47 @@ double uniform_reach(const jt_box_dev& d)
     return w * w * w;
 }
 
+// Which targets of a box the tree walk takes: those in blocks with more than
+// tot_tree particles in reach, if what it saves on them pays for building it.
+// The cell walk's time per target is that of its tot particles in reach (1.1e12
+// of them per second), the tree walk's grows with sqrt(tot) and shrinks with
+// theta (b sqrt(tot), b = 0.07 ns at theta 0.5, no less than at theta 0.8, where
+// nothing more is accepted), and a tree walk of any targets costs the trees of
+// the whole box (0.55 ns per particle) and a wave of long groups (4.5 ms at
+// theta 0.5):
+//   gain = sum n (tot - tree_cost sqrt(tot)) > gain_min     [particles in reach]
+// In a screened box the tree walk takes opposite-species pairs one by one, half
+// of what it would save.  Fitted to 19 boxes at theta 0.2 .. 1 (2x64^3 .. 2x224^3
+// particles: 4 to 512 Plummer spheres, one to 64 clumps in a uniform box), whose
+// time hardly depends on tot_tree where it does not cut through a clump.  Near
+// field of one force pass at theta 0.3 / 0.5 / 0.7, cell walk alone against the
+// tree walk above tot_tree (* what is taken):
+//   2x64^3, 64 spheres (10,700 in reach in the mean)  3.3* against 6.0 / 5.8 / 5.6 ms
+//   2x64^3, 16 spheres (24,900)      10.9* against 13.6 / 12.9 / 9.2*
+//   2x64^3, 4 spheres (83,800)       39.9 against 26.6* / 16.2* / 11.2*
+//   2x128^3, 512 spheres (9,400)     22.2* against 24.4 / 24.3 / 24.7
+//   2x128^3, 64 spheres (49,600)    162 against 146* / 99.6* / 64.0*
+//   2x128^3, a clump of 30,000        4.3* against 6.7 / 6.6 / 6.3
+//   2x128^3, a clump of 200,000      45 against 27.3* / 21.1* / 18.4*
+//   2x128^3, 8 clumps of 50,000      23.3 against 20.3* / 14.2* / 13.4*
+//   2x224^3, a clump of 100,000      21.1* against 31.8 / 29.1 / 27.6
+//   2x224^3, a clump of 500,000     256 against 236* / 146* / 96.7*
+//   screened, theta 0.5: 2x64^3, 4 spheres 41 against 22*; 2x128^3, a clump of
+//     200,000 47.1 against 48.9*, 8 clumps of 50,000 24.8* against 28.5
+// (A mean over all of the box's targets, the rule before this one, left the
+// clumps in uniform boxes to the cell walk: 45, 23 and 256 ms.)
+void tree_route(jt_box_dev& d, int64_t n, double theta, bool screened)
+{
+    const double q = 0.5 / std::min(theta, 0.8), b = std::pow(q, 0.8);   // theta 0: infinite, never
+    const double share = screened ? 0.5 : 1.0;
+    d.tree_cost = (float)(78.0 * b / share);
+    // (below tree_cost^2 the tree walk would be the slower one)
+    d.tot_tree = std::max((float)(36000.0 * std::min(q, std::sqrt(q))), d.tree_cost * d.tree_cost);
+    d.gain_min = (float)((5.0e9 * b + 610.0 * (double)n) / share);
+}
+
 // the cell list of a box with nb columns per axis
-void box_cells(jt_box_dev& d, int64_t n, int nb, const jt_config& c, double rcut)
+void box_cells(jt_box_dev& d, int64_t n, int nb, const jt_config& c, double rcut, bool screened)
 {
     const double L = c.box_L;
     d.nb = nb;
@@ -560,10 +599,7 @@ void box_cells(jt_box_dev& d, int64_t n, int nb, const jt_config& c, double rcut
     d.cellx_inv = (float)(d.nbx / L);
     // the farthest column with a gap below the cut (1e-4 margin)
     d.colm = (int)(rcut * 1.0001 * nb / L + 1.0e-4) + 1;
-    // JT_CELL_KMAX per 27 r_cut^3, in particles per bin
-    const double bin = L / nb * (L / nb) * (L / d.nbx);
-    d.cell_dmax = (float)(JT_CELL_KMAX / (27.0 * c.r_cut * c.r_cut * c.r_cut) * bin);
-    d.reach_max = (float)(JT_CELL_REACH / c.theta * (double)n);   // theta 0: no multipoles, never
+    tree_route(d, n, c.theta, screened);
     d.reach_raw = (float)(1.3 * (double)n * (double)n * uniform_reach(d));
 }
 
@@ -704,7 +740,8 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
         d.cbase = P.ncells;
         d.colbase = P.ncols;
         if (P.cells && box_has_cells(c, rcut))
-            box_cells(d, b->n[0] + b->n[1], b->cell_nb > 0 ? b->cell_nb : cell_columns(c.box_L, rcut, b->n[0] + b->n[1]), c, rcut);
+            box_cells(d, b->n[0] + b->n[1], b->cell_nb > 0 ? b->cell_nb : cell_columns(c.box_L, rcut, b->n[0] + b->n[1]), c, rcut,
+                      b->ytab != nullptr);
         P.ncells += (int64_t)d.nb * d.nb * d.nbx;
         P.ncols += (int64_t)d.nb * d.nb;
         for (int s = 0; s < 2; s++) {
@@ -771,9 +808,9 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
         JT_TRY(B->cid.ensure((size_t)std::max<int64_t>(P.npart, 1), &grew));
         JT_TRY(B->tflag.ensure((size_t)std::max<int64_t>(P.npart, 1), &grew));
         JT_TRY(B->cdense.ensure((size_t)P.ncells / 8 + 1, &grew));
-        // reach (boxes), cmap (slots), ccount (cells), segflag (segments)
+        // reach, gain (boxes), cmap (slots), ccount (cells), segflag (segments)
         const size_t slots = (size_t)(P.npart / 32 + P.ncols + 1);
-        P.o_cmap = sizeof(unsigned long long) * (size_t)nb;
+        P.o_cmap = 2 * sizeof(unsigned long long) * (size_t)nb;
         P.o_ccount = (P.o_cmap + sizeof(int2) * slots + 15) & ~(size_t)15;
         P.o_segflag = P.o_ccount + sizeof(int) * (size_t)P.ncells;
         P.cellz_bytes = P.o_segflag + sizeof(int) * (size_t)nseg;
@@ -822,6 +859,7 @@ jt_cell_bufs cell_bufs(jt_batch* B, const Plan& P)
     cb.zero = z;
     cb.zero_bytes = P.cellz_bytes;
     cb.reach = (unsigned long long*)z;
+    cb.gain = cb.reach + P.bx.size();
     cb.cmap = (int2*)(z + P.o_cmap);
     cb.ccount = (int*)(z + P.o_ccount);
     cb.segflag = (int*)(z + P.o_segflag);
@@ -871,7 +909,7 @@ int tune_cells(jt_batch* B, Plan& P, int nseg, int parts, const float4* pmacc, b
     jt_cell_bufs cb = cell_bufs(B, P);
     const cudaEvent_t e0 = B->evs[B->evi].e[8], e1 = B->evs[B->evi].e[9];   // the pass's own events around the cell walk
     auto set_nb = [&](int nb) -> int {
-        box_cells(d, bs->n[0] + bs->n[1], nb, bs->cfg, rcut);
+        box_cells(d, bs->n[0] + bs->n[1], nb, bs->cfg, rcut, false);
         P.ncols = (int64_t)nb * nb;
         P.ncells = P.ncols * d.nbx;
         if (cudaMemcpyAsync((void*)P.d_bx, &d, sizeof(jt_box_dev), cudaMemcpyHostToDevice, st) != cudaSuccess)
@@ -1567,7 +1605,7 @@ int jt_cell_layout(const jt_config* cfg, size_t n_p, size_t n_m, jt_cell_info* o
     const int64_t n = (int64_t)(n_p + n_m);
     const double rcut = jt_short_cut(*cfg);
     jt_box_dev d = {};
-    if (box_has_cells(*cfg, rcut)) box_cells(d, n, cell_columns(cfg->box_L, rcut, n), *cfg, rcut);
+    if (box_has_cells(*cfg, rcut)) box_cells(d, n, cell_columns(cfg->box_L, rcut, n), *cfg, rcut, false);
     *out = cell_layout_info(d, (double)n);
     return JT_OK;
 }

@@ -117,8 +117,10 @@ struct jt_box_dev {
     int nb;               // columns per axis (y, z) of the near-field cell list (0: tree walk only)
     int nbx;              // bins of a column along x
     int colm;             // columns in reach on either side of a batch's own (at most 2)
-    float cell_dmax;      // a block with more particles per bin in reach is dense (k_cell_dense)
-    float reach_max;      // the box's sum of particles in reach above which dense blocks go to the tree walk
+    // the tree walk for targets with many particles in reach (tree_route in jt_batch.cu)
+    float tot_tree;       // its targets have more than this in reach
+    float tree_cost;      // its time per target with tot in reach, in the cell walk's pairs: tree_cost sqrt(tot)
+    float gain_min;       // the box's gain (jt_cell_bufs) above which they go there
     float cell_inv;       // nb / L
     float cellx_inv;      // nbx / L
     float reach_raw;      // ... above which the cell walk takes differences of unscaled positions
@@ -218,22 +220,6 @@ __device__ __forceinline__ float jt_wrap(float d, float L, float halfL)
     d = (d < -halfL) ? d + L : d;
     return d;
 }
-
-// In a strongly clustered box (mean particles in reach above JT_CELL_REACH /
-// theta) the tree walk takes the targets of the blocks that have more than
-// JT_CELL_KMAX particles per 27 r_cut^3 in reach; in other boxes the cell walk
-// takes every target.  The cell walk's time grows with the particles in
-// reach, the tree walk's only as about their square root (multipoles), and
-// mixing the two in one box of middling density costs more than either
-// alone (two kernels that each wait for a few long groups).  Measured, 2x64^3
-// particles in Plummer spheres (L 50, PM 128^3, near field of one force pass),
-// by mean particles in reach, cell walk alone against tree walk:
-//   10,200 (64 spheres):  3.3 ms against 5.8 / 5.1 / 4.3 at theta 0.3 / 0.5 / 0.7
-//   28,500 (16 spheres): 10.7 ms against 13.9 / 10.8 / 8.6
-//   45,500 (2x128^3, 64 spheres): 160 ms against 147 / 99 / 64
-//   83,800 (4 spheres):  39.5 ms against 27.8 / 17.2 / 12.3
-constexpr double JT_CELL_REACH = 13500.0;
-constexpr double JT_CELL_KMAX = 2048.0;
 
 // The short-range cut of an accurate-mode box: r_cut, or with cut_tail_ppm
 // = k > 0 the radius where S(r / 2 r_s) = k * 1e-6 when that is larger.
@@ -358,10 +344,11 @@ int jt_b_walk(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t
 struct jt_cell_bufs {
     int* ccount; int* cstart; int* bsum; int* ccell; unsigned* cslot;
     float4* cpos; int2* cid; unsigned char* tflag;
-    unsigned char* dense;         // per block of 8 bins: above the tree walk's density
+    unsigned char* dense;         // per block of 8 bins: more than tot_tree in reach
+    unsigned long long* gain;     // per box: the pairs' worth of time its tree walk saves (k_cell_dense)
     unsigned long long* reach;    // per box: sum over its particles of the particles in reach
     int2* cmap;                   // batch slot -> (box + 1, column of the box), 0: none
-    // ccount, reach, cmap and segflag lie in one array, cleared by one memset
+    // ccount, reach, gain, cmap and segflag lie in one array, cleared by one memset
     void* zero;
     size_t zero_bytes;
     int* segflag;                 // per segment: some particle is flagged (its tree is built)

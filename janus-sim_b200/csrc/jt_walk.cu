@@ -1131,8 +1131,8 @@ namespace {
 // in dense chunks of 32 where every lane evaluates every candidate with the
 // pair force selected by r^2 < r_cut^2 (no per-lane hit loop, no traversal).
 // Pairs are exactly those of the tree walk when it accepts no multipole
-// (the uniform case); a strongly clustered box flags the targets of its dense
-// blocks for the tree walk, which keeps its multipoles there (k_cell_dense).
+// (the uniform case); targets with very many particles in reach are flagged
+// for the tree walk, which keeps its multipoles there (tree_route in jt_batch.cu).
 // A pass with few batches splits each among the four warps of a block
 // (jt_b_cells): every fourth column each, the sums added in shared memory.
 
@@ -1256,11 +1256,10 @@ __global__ void __launch_bounds__(kScanT) k_scan_add(int* __restrict__ out, int6
 
 // How crowded each block of 8 bins (a cube of side s) is: the particles
 // within colm blocks of it on every axis, about what its targets have in
-// reach.  cb.dense marks blocks above the tree walk's density (cell_dmax per
-// bin), cb.reach sums particles times particles in reach over each box: the
-// cost of walking all of it directly, which decides whether the box uses the
-// tree walk for its dense blocks (jt_box_dev.reach_max).  Both follow from the
-// counts alone, not from the order that the atomics gave the list.
+// reach (tot).  cb.dense marks blocks with more than tot_tree, cb.gain sums
+// over a box's targets in them what the tree walk would save, cb.reach sums tot
+// over all targets.  All follow from the counts alone, not from the order that
+// the atomics gave the list.
 // One warp per block (per consecutive blocks at large sizes: one atomic for
 // all of them), one lane per column in reach.
 __global__ void __launch_bounds__(256) k_cell_dense(const jt_box_dev* __restrict__ boxes, int nbox, int64_t nblocks,
@@ -1275,11 +1274,15 @@ __global__ void __launch_bounds__(256) k_cell_dense(const jt_box_dev* __restrict
         const int mid = (b + hi + 1) >> 1;
         if (boxes[mid].cbase <= 8 * q0) b = mid; else hi = mid - 1;
     }
-    unsigned long long work = 0;
+    unsigned long long work = 0, gain = 0;
+    const auto add_to_box = [&]() {
+        if (lane == 0 && work) atomicAdd(cb.reach + b, work);
+        if (lane == 0 && gain) atomicAdd(cb.gain + b, gain);
+        work = gain = 0;
+    };
     for (int64_t q = q0; q < q1; q++) {
         if (b + 1 < nbox && boxes[b + 1].cbase <= 8 * q) {   // into the next box (an empty grid adds no block)
-            if (lane == 0 && work) atomicAdd(cb.reach + b, work);
-            work = 0;
+            add_to_box();
             while (b + 1 < nbox && boxes[b + 1].cbase <= 8 * q) b++;
         }
         const jt_box_dev& B = boxes[b];
@@ -1302,12 +1305,13 @@ __global__ void __launch_bounds__(256) k_cell_dense(const jt_box_dev* __restrict
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-            dense = (float)tot > B.cell_dmax * (float)(8 * span * span * span);
+            dense = (float)tot > B.tot_tree;
+            if (dense) gain += (unsigned long long)((float)n * ((float)tot - B.tree_cost * sqrtf((float)tot)));
             work += (unsigned long long)n * (unsigned long long)tot;
         }
         if (lane == 0) cb.dense[q] = dense ? 1 : 0;
     }
-    if (lane == 0 && work) atomicAdd(cb.reach + b, work);
+    add_to_box();
 }
 
 // particles into cell order: (x, y, z, s m) and (segment, index; ~index for the
@@ -1326,8 +1330,8 @@ __global__ void k_cell_scatter(CellArgs A, int64_t npart)
     const float sm = SG.species == 0 ? B.mass[0] : -B.mass[1];
     const int dst = A.cb.cstart[key] + (int)A.cb.cslot[i];
     A.cb.cpos[dst] = make_float4(p.x, p.y, p.z, sm);
-    // a clustered box: the tree walk takes the targets of dense blocks
-    const bool dense = (float)A.cb.reach[SG.box] > B.reach_max && A.cb.dense[key >> 3];
+    // the targets that the tree walk takes, where they are worth building it
+    const bool dense = (float)A.cb.gain[SG.box] > B.gain_min && A.cb.dense[key >> 3];
     A.cb.cid[dst] = make_int2(g, dense ? ~(int)idx : (int)idx);
     if (dense) {
         A.cb.tflag[i] = 1;

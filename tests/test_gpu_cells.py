@@ -171,3 +171,54 @@ def test_a_small_uniform_box_is_not_clustered(n, nb):
     s.close()
     assert c["nb"] == nb and 2 * c["colm"] + 1 >= nb
     assert c["reach"] == c["reach_uniform"] == n and c["unscaled"] == 0 and c["to_tree"] == 0
+
+
+def _box_with_clumps(n, L, clumps, per, seed):
+    """n particles of one species, clumps x per / 2 of them in Gaussian clumps
+    (0.3 wide, shared by the species), the rest uniform."""
+    x = (np.random.default_rng(seed).random((n, 3)) - 0.5) * L
+    c = (np.random.default_rng(99).random((clumps, 3)) - 0.5) * 0.9 * L
+    m = clumps * per // 2
+    x[:m] = c[np.arange(m) % clumps] + np.random.default_rng(seed + 1).normal(0.0, 0.3, (m, 3))
+    return (np.remainder(x + 0.5 * L, L) - 0.5 * L).clip(-0.49999 * L, 0.49999 * L).astype(np.float32)
+
+
+# particles per species, L, PM grid, clumps, particles in each, theta, tree walk
+ROUTES = [
+    (128 ** 3, 100.0, 256, 1, 200000, 0.5, True),     # 22 ms against 45 by the cell walk
+    (128 ** 3, 100.0, 256, 1, 30000, 0.5, False),     # 4.3 ms against 6.6 by the tree walk
+    (128 ** 3, 100.0, 256, 8, 50000, 0.5, True),
+    (64 ** 3, 50.0, 128, 1, 200000, 0.0, False),      # no multipoles at theta 0
+    (64 ** 3, 50.0, 128, 1, 200000, 0.8, True),
+    (64 ** 3, 50.0, 128, 1, 1000, 0.8, False),
+]
+
+
+@pytest.mark.parametrize("n,L,M,clumps,per,theta,tree", ROUTES)
+def test_route_of_clumps_in_a_uniform_box(n, L, M, clumps, per, theta, tree):
+    """Massive clumps go to the tree walk and leave the rest of a uniform box to
+    the cell walk; the forces of both are the pairs' (targets inside and outside)."""
+    import janus_treepm as J
+    r_s = 1.25 * L / M
+    cfg = J.Config(box_L=L, pm_grid=M, theta=theta, softening=L / (2 * n) ** (1 / 3) / 30, r_s=r_s, r_cut=4.5 * r_s,
+                   mu=19.0, G_mass_plus=1.0)
+    pp, pm = _box_with_clumps(n, L, clumps, per, 1), _box_with_clumps(n, L, clumps, per, 5)
+    s = J.Solver(cfg)
+    s.set_state(pp, None, pm, None)
+    ap, am = s.accel_part(J.JT_PART_SHORT)
+    c = s.cells()
+    s.close()
+    assert (c["to_tree"] > 0) == tree and c["to_tree"] < 1.2 * clumps * per, c
+    pos = np.concatenate([pp, pm]).astype(np.float64)
+    q = np.concatenate([np.ones(n), np.full(n, -19.0)])
+    acc = np.concatenate([ap, am]).astype(np.float64)
+    rng = np.random.default_rng(0)
+    inside = rng.integers(0, clumps * per // 2, 10)
+    for t, multipoles in ((np.concatenate([inside, n + inside]), tree),
+                          (rng.integers(n - n // 8, n, 10), False)):
+        f, mag, edge = _short(pos, q, t, L, r_s, cfg.r_cut, cfg.softening)
+        err = np.linalg.norm(acc[t] - f, axis=1)
+        # the table and the sums of the cell walk (2e-5 of the magnitudes); nodes at
+        # this theta: 5e-3 of the force, 1e-4 of what the clump's pairs add up to
+        bound = 2e-5 * mag + edge + (5e-3 * np.linalg.norm(f, axis=1) + 1e-4 * mag if multipoles else 0.0)
+        assert np.all(err <= bound), (multipoles, (err / bound).max(), c)
