@@ -436,7 +436,11 @@ __device__ __forceinline__ void drain_ranges(WalkWarpSmem& S, int nr, int& nc,
 // SCR: the pass holds a screened box; the other species' tree of a screened
 // box is walked with the Yukawa table and without multipoles (their
 // expansion is of the Newtonian kernel), i.e. every pair inside r_cut
-template <bool WRAP, int BKT, bool SCR>
+//
+// Nodes of up to kBucket particles are streamed as ranges, one lane per particle
+// when a range is loaded (24 instead of 32: 8 to 20 % slower).
+constexpr int kBucket = 32;
+template <bool WRAP, bool SCR>
 __device__ __forceinline__ void walk_trees(const WalkArgs& A, const jt_box_dev& B,
                                            const jt_walk_params& P, WalkWarpSmem& S, int s, int lane,
                                            const float4& p, bool valid, float gcx, float gcy,
@@ -540,7 +544,7 @@ __device__ __forceinline__ void walk_trees(const WalkArgs& A, const jt_box_dev& 
                         }
                     }
                     if (!accepted) {
-                        if (count <= BKT) {
+                        if (count <= kBucket) {
                             act = 2;
                             rg = make_int2(first, count);
                             // shift (in box lengths) that moves the node to the group's image
@@ -639,13 +643,14 @@ __device__ __forceinline__ Acc3 pm_from_tiles(const float4* __restrict__ pmacc, 
     return Acc3{a.x, a.y, a.z};
 }
 
-// MINB: resident blocks per SM the register budget is sized for (6 -> 80
-// registers); BKT: nodes with <= BKT particles are streamed as ranges
-// (<= 32: one lane per particle when a range is loaded)
-template <int NG, int MINB, int BKT, bool SCR>
-__global__ void __launch_bounds__(kWarps * 32, MINB) k_walk_acc(WalkArgs A)
+// Resident blocks per SM that the registers are sized for: 5 (96 registers)
+// against 6 (80), whole boxes by the tree walk alone: 2x224^3 73.4 against
+// 76.3 ms, 2x160^3 24.5 against 26.1; clumps: 2x224^3 with one of 500,000
+// particles 124 against 143, 2x128^3 in 64 spheres 99.6 against 114.5.
+constexpr int kWalkMinBlocks = 5;
+template <int NG, bool SCR>
+__global__ void __launch_bounds__(kWarps * 32, kWalkMinBlocks) k_walk_acc(WalkArgs A)
 {
-    static_assert(BKT <= 32, "a range is loaded one particle per lane");
     __shared__ WalkWarpSmem smem_all[kWarps];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     WalkWarpSmem& S = smem_all[wib];
@@ -697,10 +702,10 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_walk_acc(WalkArgs A)
     // groups wider than L/8 take the minimum image per pair
     const bool wide = fmaxf(fmaxf(ghx, ghy), ghz) > 0.125f * P.L;
     if (wide)
-        walk_trees<true, BKT, SCR>(A, B, P, S, s, lane, p, valid, gcx, gcy, gcz, ghx, ghy, ghz, near,
+        walk_trees<true, SCR>(A, B, P, S, s, lane, p, valid, gcx, gcy, gcz, ghx, ghy, ghz, near,
                                     far, comp, pairs, nodes, cands, wc);
     else
-        walk_trees<false, BKT, SCR>(A, B, P, S, s, lane, p, valid, gcx, gcy, gcz, ghx, ghy, ghz, near,
+        walk_trees<false, SCR>(A, B, P, S, s, lane, p, valid, gcx, gcy, gcz, ghx, ghy, ghz, near,
                                      far, comp, pairs, nodes, cands, wc);
 
     if (valid && mine) {
@@ -1064,41 +1069,6 @@ int stab_ready()
     if (cudaMemcpyToSymbol(g_ltab, lt.data(), sizeof(float2) * JT_LTAB_N) != cudaSuccess) return JT_ECUDA;
     done[dev] = true;
     return JT_OK;
-}
-
-}  // namespace
-
-namespace {
-
-// ---- tree walk launch shapes -----------------------------------------------
-// Resident blocks per SM the registers are sized for, and the leaf bucket.
-// Boxes of up to 2^19 warp groups run best at 96 registers (5 blocks per SM),
-// larger ones at 80 (6 blocks).  (Timing the variants on a process's first
-// force pass of a size picked an arbitrary one wherever that pass sent no
-// particle to the tree walk.)  JT_WALK_VARIANT=<k> pins variant k.
-struct WalkVariant {
-    int minb, bkt;
-};
-constexpr WalkVariant kVariants[] = {{6, 32}, {5, 32}, {6, 24}};
-constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
-
-// the variants of the interlaced PM scheme
-void launch_variant(int v, unsigned g, const WalkArgs& A, cudaStream_t st)
-{
-    switch (v) {
-    case 1: k_walk_acc<2, 5, 32, false><<<g, kWarps * 32, 0, st>>>(A); break;
-    case 2: k_walk_acc<2, 6, 24, false><<<g, kWarps * 32, 0, st>>>(A); break;
-    default: k_walk_acc<2, 6, 32, false><<<g, kWarps * 32, 0, st>>>(A); break;
-    }
-}
-
-int pick_variant(int64_t ngroups)
-{
-    if (const char* e = std::getenv("JT_WALK_VARIANT")) {
-        const int v = std::atoi(e);
-        return v >= 0 && v < kNumVariants ? v : 0;
-    }
-    return ngroups <= ((int64_t)1 << 19) ? 1 : 0;
 }
 
 }  // namespace
@@ -1829,12 +1799,11 @@ int jt_b_walk(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t
     A.segflag = tflag ? segflag : nullptr;
     unsigned g = (unsigned)((ngroups + kWarps - 1) / kWarps);
     if (screened) {
-        if (ngrid == 2) k_walk_acc<2, 6, 32, true><<<g, kWarps * 32, 0, st>>>(A);
-        else k_walk_acc<1, 6, 32, true><<<g, kWarps * 32, 0, st>>>(A);
-    } else if (ngrid == 2) {
-        launch_variant(pick_variant(ngroups), g, A, st);
+        if (ngrid == 2) k_walk_acc<2, true><<<g, kWarps * 32, 0, st>>>(A);
+        else k_walk_acc<1, true><<<g, kWarps * 32, 0, st>>>(A);
     } else {
-        k_walk_acc<1, 6, 32, false><<<g, kWarps * 32, 0, st>>>(A);
+        if (ngrid == 2) k_walk_acc<2, false><<<g, kWarps * 32, 0, st>>>(A);
+        else k_walk_acc<1, false><<<g, kWarps * 32, 0, st>>>(A);
     }
     return cudaGetLastError() == cudaSuccess ? JT_OK : JT_ECUDA;
 }
