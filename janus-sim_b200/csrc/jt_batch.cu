@@ -600,7 +600,11 @@ void box_cells(jt_box_dev& d, int64_t n, int nb, const jt_config& c, double rcut
     // the farthest column with a gap below the cut (1e-4 margin)
     d.colm = (int)(rcut * 1.0001 * nb / L + 1.0e-4) + 1;
     tree_route(d, n, c.theta, screened);
+    // clustered: 1.3 times a uniform box's particles in reach on average, or twice
+    // somewhere (a clump in a uniform box; the largest count of a uniform box is
+    // 1.2 times the mean: 860 particles and more, Poisson)
     d.reach_raw = (float)(1.3 * (double)n * (double)n * uniform_reach(d));
+    d.tot_crowd = (float)(2.0 * (double)n * uniform_reach(d));
 }
 
 // whether the box has a cell list (at least three cuts along it), and its layout
@@ -945,7 +949,7 @@ int tune_cells(jt_batch* B, Plan& P, int nseg, int parts, const float4* pmacc, b
             // particles in reach twice that of a uniform box): keep it
             if (r == JT_OK && nb == nmax) {
                 const double n = (double)(bs->n[0] + bs->n[1]);
-                crowded = flag[0] || flag[1] || (double)reach > 2.0 * n * n * uniform_reach(d);
+                crowded = flag[0] || flag[1] || (double)(reach & ~JT_REACH_CROWD) > 2.0 * n * n * uniform_reach(d);
                 if (crowded) {
                     if (!B->counters) {
                         B->tm.pair_interactions += (int64_t)count[0];
@@ -1179,7 +1183,7 @@ int jtb_cell_info(jt_batch* B, jt_cell_info* out)
     JT_CU(cudaMemcpyAsync(flags.data(), cb.tflag, flags.size(), cudaMemcpyDeviceToHost, B->st));
     JT_CU(cudaStreamSynchronize(B->st));
     for (unsigned char f : flags) out->to_tree += f ? 1 : 0;
-    out->reach = (double)reach / (double)P.npart;
+    out->reach = (double)(reach & ~JT_REACH_CROWD) / (double)P.npart;
     out->unscaled = (float)reach > d.reach_raw ? 1 : 0;
     return JT_OK;
 }

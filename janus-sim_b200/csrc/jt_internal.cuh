@@ -123,7 +123,9 @@ struct jt_box_dev {
     float gain_min;       // the box's gain (jt_cell_bufs) above which they go there
     float cell_inv;       // nb / L
     float cellx_inv;      // nbx / L
-    float reach_raw;      // ... above which the cell walk takes differences of unscaled positions
+    // a clustered box's cell walk takes differences of unscaled positions:
+    float reach_raw;      // its sum of particles in reach (jt_cell_bufs) is above this, or
+    float tot_crowd;      // it has a crowded block, with more than this in reach
     int64_t cbase;        // this box's first cell in the pass's cell tables
     int64_t colbase;      // this box's first column in the pass
 };
@@ -341,12 +343,15 @@ int jt_b_walk(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t
 // ints, bsum, cmap nslots, dense ncells / 8, reach nbox, ccell/cslot, cpos/cid
 // one entry per particle.
 // nslots: npart / 32 + the columns of all boxes.
+constexpr unsigned long long JT_REACH_CROWD = 1ull << 63;
 struct jt_cell_bufs {
     int* ccount; int* cstart; int* bsum; int* ccell; unsigned* cslot;
     float4* cpos; int2* cid; unsigned char* tflag;
     unsigned char* dense;         // per block of 8 bins: more than tot_tree in reach
     unsigned long long* gain;     // per box: the pairs' worth of time its tree walk saves (k_cell_dense)
-    unsigned long long* reach;    // per box: sum over its particles of the particles in reach
+    // per box: sum over its particles of the particles in reach, and the bit
+    // JT_REACH_CROWD if it has a crowded block
+    unsigned long long* reach;
     int2* cmap;                   // batch slot -> (box + 1, column of the box), 0: none
     // ccount, reach, gain, cmap and segflag lie in one array, cleared by one memset
     void* zero;

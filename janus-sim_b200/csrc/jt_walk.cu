@@ -1228,8 +1228,8 @@ __global__ void __launch_bounds__(kScanT) k_scan_add(int* __restrict__ out, int6
 // within colm blocks of it on every axis, about what its targets have in
 // reach (tot).  cb.dense marks blocks with more than tot_tree, cb.gain sums
 // over a box's targets in them what the tree walk would save, cb.reach sums tot
-// over all targets.  All follow from the counts alone, not from the order that
-// the atomics gave the list.
+// over all targets and marks a box with a crowded block (above tot_crowd).  All
+// follow from the counts alone, not from the order that the atomics gave the list.
 // One warp per block (per consecutive blocks at large sizes: one atomic for
 // all of them), one lane per column in reach.
 __global__ void __launch_bounds__(256) k_cell_dense(const jt_box_dev* __restrict__ boxes, int nbox, int64_t nblocks,
@@ -1245,8 +1245,11 @@ __global__ void __launch_bounds__(256) k_cell_dense(const jt_box_dev* __restrict
         if (boxes[mid].cbase <= 8 * q0) b = mid; else hi = mid - 1;
     }
     unsigned long long work = 0, gain = 0;
+    bool crowd = false;
     const auto add_to_box = [&]() {
         if (lane == 0 && work) atomicAdd(cb.reach + b, work);
+        if (lane == 0 && crowd) atomicOr(cb.reach + b, JT_REACH_CROWD);
+        crowd = false;
         if (lane == 0 && gain) atomicAdd(cb.gain + b, gain);
         work = gain = 0;
     };
@@ -1275,6 +1278,7 @@ __global__ void __launch_bounds__(256) k_cell_dense(const jt_box_dev* __restrict
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+            crowd = crowd || (float)tot > B.tot_crowd;
             dense = (float)tot > B.tot_tree;
             if (dense) gain += (unsigned long long)((float)n * ((float)tot - B.tree_cost * sqrtf((float)tot)));
             work += (unsigned long long)n * (unsigned long long)tot;
@@ -1545,7 +1549,7 @@ __global__ void __launch_bounds__(kWarps * 32, kCellMinBlocks) k_walk_cell(CellA
         }
         __syncwarp();
         if ((A.parts & 2) && nr > 0) {
-            const bool raw = (float)A.cb.reach[where.x - 1] > B.reach_raw;
+            const bool raw = (float)A.cb.reach[where.x - 1] > B.reach_raw;   // JT_REACH_CROWD is above any
             const float ps = raw ? 1.0f : cc;   // what positions are scaled by
             // the filter's uniform values live in shared memory: they are read
             // once per 32 candidates and would spill the pair loop's registers

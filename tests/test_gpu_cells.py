@@ -222,3 +222,32 @@ def test_route_of_clumps_in_a_uniform_box(n, L, M, clumps, per, theta, tree):
         # this theta: 5e-3 of the force, 1e-4 of what the clump's pairs add up to
         bound = 2e-5 * mag + edge + (5e-3 * np.linalg.norm(f, axis=1) + 1e-4 * mag if multipoles else 0.0)
         assert np.all(err <= bound), (multipoles, (err / bound).max(), c)
+
+
+def test_a_dense_clump_in_a_uniform_box_keeps_its_digits():
+    """Targets inside a clump too small for the tree walk and for the box's mean to
+    call it clustered: their differences are of unscaled positions and their sums
+    run in chunks (scaled positions and running sums: 5e-5 of the force)."""
+    import janus_treepm as J
+    n, L, M, k = 64 ** 3, 50.0, 128, 12000
+    r_s = 1.25 * L / M
+    cfg = J.Config(box_L=L, pm_grid=M, softening=L / (2 * n) ** (1 / 3) / 30, r_s=r_s, r_cut=4.5 * r_s, mu=1.0,
+                   G_mass_plus=1.0)
+    pts = []
+    for seed in (1, 2):
+        x = (np.random.default_rng(seed).random((n, 3)) - 0.5) * L
+        x[:k] = [20.3, -21.7, 19.1] + np.random.default_rng(seed + 10).normal(0.0, 0.1, (k, 3))
+        pts.append(x.astype(np.float32))
+    s = J.Solver(cfg)
+    s.set_state(pts[0], None, pts[1], None)
+    ap, _ = s.accel_part(J.JT_PART_SHORT)
+    c = s.cells()
+    s.close()
+    assert c["to_tree"] == 0 and c["reach"] < 1.3 * c["reach_uniform"] and c["unscaled"] == 1, c
+    pos = np.concatenate(pts).astype(np.float64)
+    q = np.concatenate([np.ones(n), -np.ones(n)])
+    t = np.arange(0, k, k // 60)
+    f, mag, _ = _short(pos, q, t, L, r_s, cfg.r_cut, cfg.softening)
+    err = np.linalg.norm(ap[t] - f) / np.linalg.norm(f)
+    # each pair rounded once or twice (2^-24), the table without bias; 1e-5 here
+    assert err < 2.0 * 2.0 ** -24 * np.linalg.norm(mag) / np.linalg.norm(f), err
