@@ -343,11 +343,13 @@ int jt_b_walk(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t
 // ints, bsum, cmap nslots, dense ncells / 8, reach nbox, ccell/cslot, cpos/cid
 // one entry per particle.
 // nslots: npart / 32 + the columns of all boxes.
+constexpr unsigned char JT_BLOCK_TREE = 1;    // more than tot_tree in reach
+constexpr unsigned char JT_BLOCK_CROWD = 2;   // more than tot_crowd in reach
 constexpr unsigned long long JT_REACH_CROWD = 1ull << 63;
 struct jt_cell_bufs {
     int* ccount; int* cstart; int* bsum; int* ccell; unsigned* cslot;
     float4* cpos; int2* cid; unsigned char* tflag;
-    unsigned char* dense;         // per block of 8 bins: more than tot_tree in reach
+    unsigned char* dense;         // per block of 8 bins: JT_BLOCK_* bits
     unsigned long long* gain;     // per box: the pairs' worth of time its tree walk saves (k_cell_dense)
     // per box: sum over its particles of the particles in reach, and the bit
     // JT_REACH_CROWD if it has a crowded block

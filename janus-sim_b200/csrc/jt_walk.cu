@@ -1226,9 +1226,9 @@ __global__ void __launch_bounds__(kScanT) k_scan_add(int* __restrict__ out, int6
 
 // How crowded each block of 8 bins (a cube of side s) is: the particles
 // within colm blocks of it on every axis, about what its targets have in
-// reach (tot).  cb.dense marks blocks with more than tot_tree, cb.gain sums
-// over a box's targets in them what the tree walk would save, cb.reach sums tot
-// over all targets and marks a box with a crowded block (above tot_crowd).  All
+// reach (tot).  cb.dense marks blocks above tot_tree and crowded ones (above
+// tot_crowd), cb.gain sums over a box's targets above tot_tree what the tree walk
+// would save, cb.reach sums tot over all and marks a box with a crowded block.  All
 // follow from the counts alone, not from the order that the atomics gave the list.
 // One warp per block (per consecutive blocks at large sizes: one atomic for
 // all of them), one lane per column in reach.
@@ -1263,7 +1263,7 @@ __global__ void __launch_bounds__(256) k_cell_dense(const jt_box_dev* __restrict
         const int* __restrict__ cstart = cb.cstart + B.cbase;
         const int64_t local = q - B.cbase / 8;
         const int n = cstart[8 * local + 8] - cstart[8 * local];
-        bool dense = false;
+        unsigned char marks = 0;
         if (n > 0) {
             const int kx = (int)(local % nb), cy = (int)((local / nb) % nb), cz = (int)(local / ((int64_t)nb * nb));
             const int span = min(w, nb);   // blocks per axis: each of a small box's once
@@ -1278,12 +1278,17 @@ __global__ void __launch_bounds__(256) k_cell_dense(const jt_box_dev* __restrict
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-            crowd = crowd || (float)tot > B.tot_crowd;
-            dense = (float)tot > B.tot_tree;
-            if (dense) gain += (unsigned long long)((float)n * ((float)tot - B.tree_cost * sqrtf((float)tot)));
+            if ((float)tot > B.tot_crowd) {
+                marks |= JT_BLOCK_CROWD;
+                crowd = true;
+            }
+            if ((float)tot > B.tot_tree) {
+                marks |= JT_BLOCK_TREE;
+                gain += (unsigned long long)((float)n * ((float)tot - B.tree_cost * sqrtf((float)tot)));
+            }
             work += (unsigned long long)n * (unsigned long long)tot;
         }
-        if (lane == 0) cb.dense[q] = dense ? 1 : 0;
+        if (lane == 0) cb.dense[q] = marks;
     }
     add_to_box();
 }
@@ -1305,7 +1310,7 @@ __global__ void k_cell_scatter(CellArgs A, int64_t npart)
     const int dst = A.cb.cstart[key] + (int)A.cb.cslot[i];
     A.cb.cpos[dst] = make_float4(p.x, p.y, p.z, sm);
     // the targets that the tree walk takes, where they are worth building it
-    const bool dense = (float)A.cb.gain[SG.box] > B.gain_min && A.cb.dense[key >> 3];
+    const bool dense = (float)A.cb.gain[SG.box] > B.gain_min && (A.cb.dense[key >> 3] & JT_BLOCK_TREE);
     A.cb.cid[dst] = make_int2(g, dense ? ~(int)idx : (int)idx);
     if (dense) {
         A.cb.tflag[i] = 1;
@@ -1382,7 +1387,8 @@ struct CellTarget {
 // Two candidates' forces into the lane's sums, one after the other: the sums
 // run in the list's order whatever the filter of the batch let through (what
 // it drops would add exactly 0), so that two targets at one point get the same
-// bits in different batches of a column.
+// bits in different batches of a column, unless their block is crowded (then
+// chunks of the list are summed on their own, see k_walk_cell).
 __device__ __forceinline__ void add_pair(CellTarget& T, f32x2 w, f32x2 dx, f32x2 dy, f32x2 dz)
 {
     const float2 ww = unpack2(w), x = unpack2(dx), y = unpack2(dy), z = unpack2(dz);
@@ -1551,6 +1557,10 @@ __global__ void __launch_bounds__(kWarps * 32, kCellMinBlocks) k_walk_cell(CellA
         if ((A.parts & 2) && nr > 0) {
             const bool raw = (float)A.cb.reach[where.x - 1] > B.reach_raw;   // JT_REACH_CROWD is above any
             const float ps = raw ? 1.0f : cc;   // what positions are scaled by
+            // this lane's target lies in a crowded block: its sum is cut into chunks
+            const bool chunked =
+                raw && (A.cb.dense[(B.cbase + (int64_t)col * nbx + cell_of(p.x, B.halfL, B.cellx_inv, nbx)) >> 3] &
+                        JT_BLOCK_CROWD);
             // the filter's uniform values live in shared memory: they are read
             // once per 32 candidates and would spill the pair loop's registers
             if (lane == 0) {
@@ -1603,11 +1613,12 @@ __global__ void __launch_bounds__(kWarps * 32, kCellMinBlocks) k_walk_cell(CellA
                 if (nc >= 32) {
                     hits += cell_chunk<SCR, CNT>(S, 32, T, yt);
                     cands += 32;
-                    if (raw) {
+                    if (chunked) {
                         // the list runs through a clump from one side to the
                         // other, so a sum of its tens of thousands of pairs
                         // passes far above its end: chunks are summed on their
-                        // own (error in overlapping clumps 1.3e-5 -> 2.8e-6 of the force)
+                        // own (error in overlapping clumps 1.3e-5 -> 2.8e-6 of the
+                        // force).  Where chunks end depends on the batch.
                         near.x += T.ax;
                         near.y += T.ay;
                         near.z += T.az;

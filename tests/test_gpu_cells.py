@@ -251,3 +251,28 @@ def test_a_dense_clump_in_a_uniform_box_keeps_its_digits():
     err = np.linalg.norm(ap[t] - f) / np.linalg.norm(f)
     # each pair rounded once or twice (2^-24), the table without bias; 1e-5 here
     assert err < 2.0 * 2.0 ** -24 * np.linalg.norm(mag) / np.linalg.norm(f), err
+
+
+def test_opposite_species_at_one_point_in_a_clustered_box():
+    """An m- particle on top of every m+ one takes exactly the opposite
+    acceleration outside the crowded blocks, whichever batch either is in; inside,
+    to the rounding of sums cut at different places."""
+    import janus_treepm as J
+    n, L, k = 60000, 40.0, 24000
+    rng = np.random.default_rng(7)
+    x = (rng.random((n, 3)) - 0.5) * L
+    x[:k] = [12.0, 11.0, -13.0] + rng.normal(0.0, 0.8, (k, 3))
+    x = x.astype(np.float32)
+    s = J.Solver(J.Config(box_L=L, pm_grid=64, mu=3.0, softening=0.02))
+    s.set_state(x, None, x.copy(), None)
+    ap, am = s.accel_part(J.JT_PART_SHORT)
+    c = s.cells()
+    s.close()
+    assert c["unscaled"] == 1 and c["to_tree"] == 0, c
+    # blocks whose reach misses the clump (5 standard deviations and a block's side more)
+    side = L / c["nb"]
+    d = np.abs(x.astype(np.float64) - [12.0, 11.0, -13.0])
+    far = (np.minimum(d, L - d) > (c["colm"] + 2) * side + 4.0).any(1)
+    assert far.sum() > 10000
+    assert np.array_equal(am[far], -ap[far]), (am[far] != -ap[far]).any(1).sum()
+    assert np.abs(am + ap).max() <= 1e-5 * np.abs(ap).max()
