@@ -1423,8 +1423,8 @@ __device__ __forceinline__ void ld_inside(float2& ab, const float2* __restrict__
 // instruction per candidate, off unless the caller asks for them).
 // y = r^2 c^2 + ye (c = 1 / (2 r_s), ye = eps^2 c^2), and the pair is inside
 // the cut for y < yc.  Positions come scaled by c (T.c2 = 1) except in
-// clustered boxes (T.c2 = c^2), where the scaling's rounding, of the size of a
-// coordinate's ulp, would set the error of close pairs: 1e-5 of the force
+// clustered boxes (by a power of two, T.c2 the rest of c^2), where the scaling's
+// rounding, of the size of a coordinate's ulp, would set the error of close pairs: 1e-5 of the force
 // inside a clump against 1.5e-6.  (A second loop without T.c2 for the scaled
 // boxes, half a slot per candidate less, measured no faster.)  No clamp on
 // the table index: the caller bounds ye >= 2^-32 and yc < 64, so that every
@@ -1556,7 +1556,10 @@ __global__ void __launch_bounds__(kWarps * 32, kCellMinBlocks) k_walk_cell(CellA
         __syncwarp();
         if ((A.parts & 2) && nr > 0) {
             const bool raw = (float)A.cb.reach[where.x - 1] > B.reach_raw;   // JT_REACH_CROWD is above any
-            const float ps = raw ? 1.0f : cc;   // what positions are scaled by
+            // what positions are scaled by: c, or the power of two below it, which
+            // rounds nothing (and keeps the squares of any box's lengths in range)
+            const float ps = raw ? __uint_as_float(__float_as_uint(cc) & 0x7f800000u) : cc;
+            const float cps = cc / ps;   // 1, or c over that power of two
             // this lane's target lies in a crowded block: its sum is cut into chunks
             const bool chunked =
                 raw && (A.cb.dense[(B.cbase + (int64_t)col * nbx + cell_of(p.x, B.halfL, B.cellx_inv, nbx)) >> 3] &
@@ -1575,7 +1578,7 @@ __global__ void __launch_bounds__(kWarps * 32, kCellMinBlocks) k_walk_cell(CellA
             T.ny = pack2(-p.y * ps, -p.y * ps);
             T.nz = pack2(-p.z * ps, -p.z * ps);
             T.ye = pack2(ye, ye);
-            T.c2 = raw ? pack2(c2, c2) : pack2(1.0f, 1.0f);
+            T.c2 = pack2(cps * cps, cps * cps);
             T.si = si;
             T.yc = fminf(fmaf(B.rc2, c2, ye), 64.0f * 0.99999f);
             T.ax = T.ay = T.az = 0.0f;
@@ -1652,7 +1655,7 @@ __global__ void __launch_bounds__(kWarps * 32, kCellMinBlocks) k_walk_cell(CellA
                 hits += cell_chunk<SCR, CNT>(S, (nc + 3) & ~3, T, yt);
                 cands += nc;
             }
-            const float sc = si * c2 * (raw ? cc : 1.0f);   // sum w d, d scaled by ps
+            const float sc = si * c2 * cps;   // sum w d, d scaled by ps
             near = Acc3{(near.x + T.ax) * sc, (near.y + T.ay) * sc, (near.z + T.az) * sc};
         }
     }

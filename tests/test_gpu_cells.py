@@ -276,3 +276,24 @@ def test_opposite_species_at_one_point_in_a_clustered_box():
     assert far.sum() > 10000
     assert np.array_equal(am[far], -ap[far]), (am[far] != -ap[far]).any(1).sum()
     assert np.abs(am + ap).max() <= 1e-5 * np.abs(ap).max()
+
+
+def test_a_clustered_box_of_any_length_unit():
+    """The same clustered box in units 2^57 times smaller (L = 5.8e18): the
+    accelerations, scaled back, are the same up to the order of the sums."""
+    import janus_treepm as J
+    out = []
+    for e in (0, 57):
+        u = 2.0 ** e
+        L = 40.0 * u
+        x = [_points("clump", 4000, 40.0, seed) * np.float32(u) for seed in (1, 2)]
+        cfg = J.Config(box_L=L, pm_grid=32, softening=0.02 * u, r_s=1.25 * L / 32, r_cut=4.5 * 1.25 * L / 32, mu=3.0,
+                       G_mass_plus=2.0 ** (2 * e - 40 if e else 0))
+        s = J.Solver(cfg)
+        s.set_state(x[0], None, x[1], None)
+        acc = np.concatenate(s.accel_part(J.JT_PART_SHORT)).astype(np.float64)
+        assert s.cells()["unscaled"] == 1 and s.cells()["to_tree"] == 0
+        s.close()
+        out.append(acc * (2.0 ** 40 if e else 1.0))
+    assert np.isfinite(out[1]).all()
+    assert np.abs(out[1] - out[0]).max() <= 1e-5 * np.abs(out[0]).max()
