@@ -381,6 +381,9 @@ typedef struct jt_cell_info {
 } jt_cell_info;
 int  jt_cell_layout(const jt_config* cfg, size_t n_p, size_t n_m, jt_cell_info* out);
 int  jt_debug_cells(jt_handle* h, jt_cell_info* out);
+/* The slot that batch `batch` (32 particles) of a column takes in a pass's batch
+ * table, for a column that starts at particle `start` of the cell list. */
+int  jt_cell_slot(int64_t start, int64_t column, int64_t batch, int64_t* slot);
 /* Tests of the failure path, host side only: set the error word of an
  * accurate-mode handle as a walk-stack overflow (JT_EOVERFLOW) or a sort
  * time-out (JT_ETIMEDOUT) would, or let its next force pass fail on the host
@@ -469,7 +472,9 @@ int  jt_batch_box_info(jt_batch* b, int box_id, size_t* n_p, size_t* n_m, size_t
 /* Device bytes held: persistent box state, and the grow-only per-pass scratch. */
 int  jt_batch_memory(jt_batch* b, size_t* persistent, size_t* scratch);
 /* Device bytes one box would need (no device work): its persistent state and
- * its share of the per-pass scratch.  The serving loop's admission control. */
+ * its share of the per-pass scratch.  The serving loop's admission control.
+ * For an unscreened box: one with jt_batch_set_screening on takes its grids and
+ * 16 bytes per particle and interlaced grid once more. */
 int  jt_batch_estimate(const jt_config* cfg, size_t n_p, size_t n_m,
                        size_t* persistent, size_t* scratch);
 int  jt_batch_get_timings(jt_batch* b, jt_timings* t);

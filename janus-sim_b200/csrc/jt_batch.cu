@@ -566,17 +566,17 @@ double uniform_reach(const jt_box_dev& d)
 // field of one force pass at theta 0.3 / 0.5 / 0.7, cell walk alone against the
 // tree walk above tot_tree (* what is taken):
 //   2x64^3, 64 spheres (10,700 in reach in the mean)  3.3* against 6.0 / 5.8 / 5.6 ms
-//   2x64^3, 16 spheres (24,900)      10.9* against 13.6 / 12.9 / 9.2*
-//   2x64^3, 4 spheres (83,800)       39.9 against 26.6* / 16.2* / 11.2*
-//   2x128^3, 512 spheres (9,400)     22.2* against 24.4 / 24.3 / 24.7
-//   2x128^3, 64 spheres (49,600)    162 against 146* / 99.6* / 64.0*
+//   2x64^3, 16 spheres (24,900)      10.7* against 13.5 / 13.2 / 8.9*
+//   2x64^3, 4 spheres (83,800)       39.7 against 26.6* / 16.1* / 11.1*
+//   2x128^3, 512 spheres (9,400)     22.1* against 24.4 / 24.3 / 24.7
+//   2x128^3, 64 spheres (49,600)    161 against 147* / 99.6* / 64.1*
 //   2x128^3, a clump of 30,000        4.3* against 6.7 / 6.6 / 6.3
-//   2x128^3, a clump of 200,000      45 against 27.3* / 21.1* / 18.4*
-//   2x128^3, 8 clumps of 50,000      23.3 against 20.3* / 14.2* / 13.4*
-//   2x224^3, a clump of 100,000      21.1* against 31.8 / 29.1 / 27.6
-//   2x224^3, a clump of 500,000     256 against 236* / 146* / 96.7*
-//   screened, theta 0.5: 2x64^3, 4 spheres 41 against 22*; 2x128^3, a clump of
-//     200,000 47.1 against 48.9*, 8 clumps of 50,000 24.8* against 28.5
+//   2x128^3, a clump of 200,000      44 against 28.1* / 21.4* / 18.2*
+//   2x128^3, 8 clumps of 50,000      23.2 against 20.5* / 14.2* / 13.4*
+//   2x224^3, a clump of 100,000      21.1* against 29.7 / 25.9 / 24.5
+//   2x224^3, a clump of 500,000     255 against 207* / 125* / 77.7*
+//   screened, theta 0.5: 2x64^3, 4 spheres 41.1 against 16.7*; 2x128^3, a clump
+//     of 200,000 46.1 against 40.6*, 8 clumps of 50,000 24.7* against 23.2
 // (A mean over all of the box's targets, the rule before this one, left the
 // clumps in uniform boxes to the cell walk: 45, 23 and 256 ms.)
 void tree_route(jt_box_dev& d, int64_t n, double theta, bool screened)
@@ -813,7 +813,7 @@ int build_plan(jt_batch* B, const std::vector<int>& ids, const jt_box_step* step
         JT_TRY(B->tflag.ensure((size_t)std::max<int64_t>(P.npart, 1), &grew));
         JT_TRY(B->cdense.ensure((size_t)P.ncells / 8 + 1, &grew));
         // reach, gain (boxes), cmap (slots), ccount (cells), segflag (segments)
-        const size_t slots = (size_t)(P.npart / 32 + P.ncols + 1);
+        const size_t slots = (size_t)jt_slot(P.npart, P.ncols, 0) + 1;
         P.o_cmap = 2 * sizeof(unsigned long long) * (size_t)nb;
         P.o_ccount = (P.o_cmap + sizeof(int2) * slots + 15) & ~(size_t)15;
         P.o_segflag = P.o_ccount + sizeof(int) * (size_t)P.ncells;
@@ -932,7 +932,7 @@ int tune_cells(jt_batch* B, Plan& P, int nseg, int parts, const float4* pmacc, b
         int flag[2] = {0, 0};
         unsigned long long reach = 0, count[3] = {0, 0, 0};
         for (int rep = 0; rep < 2 && r == JT_OK; rep++) {
-            r = jt_b_cells(P.d_post, P.d_bx, P.d_pp, nseg, P.npart, 1, P.ncells, P.npart / 32 + P.ncols, cb,
+            r = jt_b_cells(P.d_post, P.d_bx, P.d_pp, nseg, P.npart, 1, P.ncells, jt_slot(P.npart, P.ncols, 0), cb,
                            B->ngrid, parts, 0.0f, stats, B->d_err, st, e0, e1, false, pmacc, false);
             if (r == JT_OK && (cudaMemcpyAsync(flag, cb.segflag, sizeof(int) * (size_t)nseg,
                                                cudaMemcpyDeviceToHost, st) != cudaSuccess ||
@@ -1063,7 +1063,7 @@ int force_pass(jt_batch* B, Plan& P, int parts, float kick_frac)
         const jt_cell_bufs cb = cell_bufs(B, P);
         if (!done)
             JT_TRY(jt_b_cells(P.d_post, P.d_bx, P.d_pp, nseg, P.npart, nbox, P.ncells,
-                              P.ncells > 0 ? P.npart / 32 + P.ncols : 0, cb, B->ngrid, parts, kick_frac,
+                              P.ncells > 0 ? jt_slot(P.npart, P.ncols, 0) : 0, cb, B->ngrid, parts, kick_frac,
                               B->d_stats, B->d_err, st, ev[8], ev[9], P.screened, pmacc, B->counters));
         tflag = B->tflag.p;
         jt_b_build_trees(P.d_post, P.d_bx, nseg, P.d_ip, P.ninternal, P.d_pp, P.npart, st, cb.segflag);
@@ -1611,6 +1611,13 @@ int jt_cell_layout(const jt_config* cfg, size_t n_p, size_t n_m, jt_cell_info* o
     jt_box_dev d = {};
     if (box_has_cells(*cfg, rcut)) box_cells(d, n, cell_columns(cfg->box_L, rcut, n), *cfg, rcut, false);
     *out = cell_layout_info(d, (double)n);
+    return JT_OK;
+}
+
+int jt_cell_slot(int64_t start, int64_t column, int64_t batch, int64_t* slot)
+{
+    if (!slot || start < 0 || column < 0 || batch < 0) return JT_EINVAL;
+    *slot = jt_slot(start, column, batch);
     return JT_OK;
 }
 

@@ -342,7 +342,12 @@ int jt_b_walk(const jt_seg_dev* d_segs, const jt_box_dev* d_boxes, const int64_t
 // acceleration (and fused kick) here.  Scratch: ccount/cstart ncells + 1
 // ints, bsum, cmap nslots, dense ncells / 8, reach nbox, ccell/cslot, cpos/cid
 // one entry per particle.
-// nslots: npart / 32 + the columns of all boxes.
+// The slot of a column's batch k in cmap.  A column c (counted over the pass's
+// boxes) that starts at particle `start` of the list owns the slots from start /
+// 32 + c: the next column's first slot lies at least ceil(count / 32) further, so
+// no prefix sum of batch counts is needed, and all columns' slots end at
+// jt_slot(npart, ncols, 0).
+__host__ __device__ inline int64_t jt_slot(int64_t start, int64_t column, int64_t k) { return (start >> 5) + column + k; }
 constexpr unsigned char JT_BLOCK_TREE = 1;    // more than tot_tree in reach
 constexpr unsigned char JT_BLOCK_CROWD = 2;   // more than tot_crowd in reach
 constexpr unsigned long long JT_REACH_CROWD = 1ull << 63;

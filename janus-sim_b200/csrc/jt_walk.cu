@@ -1318,13 +1318,10 @@ __global__ void k_cell_scatter(CellArgs A, int64_t npart)
         if (B.seg[0] >= 0) A.cb.segflag[B.seg[0]] = 1;
         if (B.seg[1] >= 0) A.cb.segflag[B.seg[1]] = 1;
     }
-    // the first particle of each batch of 32 enters the batch in cmap.  A
-    // column c (counted over the pass's boxes) that starts at particle t0
-    // owns the slots from t0 / 32 + c: the next column's first slot lies at
-    // least ceil(count / 32) further, so no prefix sum of batch counts is needed
+    // the first particle of each batch of 32 enters the batch in cmap
     const int col = (int)((key - B.cbase) / B.nbx);
     const int t0 = A.cb.cstart[B.cbase + (int64_t)col * B.nbx];
-    if (((dst - t0) & 31) == 0) A.cb.cmap[(t0 >> 5) + B.colbase + col + ((dst - t0) >> 5)] = make_int2(SG.box + 1, col);
+    if (((dst - t0) & 31) == 0) A.cb.cmap[jt_slot(t0, B.colbase + col, (dst - t0) >> 5)] = make_int2(SG.box + 1, col);
 }
 
 constexpr int kCellRanges = 75;   // 25 columns, each with up to 3 images along x
@@ -1491,7 +1488,7 @@ __global__ void __launch_bounds__(kWarps * 32, kCellMinBlocks) k_walk_cell(CellA
     const int nb = B.nb, nbx = B.nbx, col = where.y;
     const int* __restrict__ cstart = A.cb.cstart + B.cbase;
     const int tc = cstart[(int64_t)col * nbx], t1 = cstart[(int64_t)(col + 1) * nbx];
-    const int t0 = tc + 32 * (int)(slot - ((tc >> 5) + B.colbase + col));
+    const int t0 = tc + 32 * (int)(slot - jt_slot(tc, B.colbase + col, 0));
     // an index below 0 marks a target of the tree walk (k_cell_scatter); a lane
     // without a target of its own evaluates the batch's first that has one
     const unsigned live = __ballot_sync(0xffffffffu, t0 + lane < t1 && A.cb.cid[t0 + lane].y >= 0);

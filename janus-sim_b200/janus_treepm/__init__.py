@@ -45,7 +45,8 @@ EXPORTED = [
     "jt_batch_trim", "jt_batch_set_graphs", "jt_server_create", "jt_server_destroy",
     "jt_server_add_job", "jt_server_request", "jt_server_clock", "jt_server_poll", "jt_server_serve",
     "jt_server_job_state", "jt_server_get_state", "jt_server_stats", "jt_server_job_need",
-    "jt_walk_tuning", "jt_wait_probe", "jt_inject_error", "jt_cell_layout", "jt_debug_cells", "jt_diagnostics", "jt_batch_diagnostics",
+    "jt_walk_tuning", "jt_wait_probe", "jt_inject_error", "jt_cell_layout", "jt_debug_cells", "jt_cell_slot",
+    "jt_diagnostics", "jt_batch_diagnostics",
     "jt_snapshot_write", "jt_snapshot_read", "jt_checkpoint", "jt_set_screening",
     "jt_ics_zeldovich", "jt_set_state_zeldovich", "jt_batch_add_zeldovich", "jt_philox4x32_10",
     "jt_energy_sampled", "jt_virialize_sampled", "jt_energy_drift_pct",
@@ -309,6 +310,7 @@ def library():
     L.jt_inject_error.argtypes = [H, C.c_int]
     L.jt_cell_layout.argtypes = [C.POINTER(jt_config), C.c_size_t, C.c_size_t, C.POINTER(jt_cell_info)]
     L.jt_debug_cells.argtypes = [H, C.POINTER(jt_cell_info)]
+    L.jt_cell_slot.argtypes = [C.c_int64, C.c_int64, C.c_int64, C.POINTER(C.c_int64)]
     L.jt_wait_probe.argtypes = [C.c_int, C.POINTER(C.c_int)]
     L.jt_diagnostics.argtypes = [H, C.c_int, C.POINTER(jt_diag)]
     L.jt_snapshot_write.argtypes = [C.c_char_p, C.POINTER(jt_snapshot_meta), C.c_double, C.c_double,

@@ -24,8 +24,9 @@ def _erfc(x):
 
 
 def _short(pos, q, targets, L, r_s, rc, eps):
-    """(force, sum of |pair force|, what pairs within 1e-5 of the cut carry)."""
-    out, mag, edge = [], [], []
+    """(force, sum of |pair force|, what pairs within 1e-5 of the cut carry, sum of
+    |pair force| / r_p, pairs), per target."""
+    out, mag, edge, grad, cnt = [], [], [], [], []
     for t in targets:
         d = pos - pos[t]
         d -= L * np.round(d / L)
@@ -40,7 +41,18 @@ def _short(pos, q, targets, L, r_s, rc, eps):
         out.append((f[~at_cut, None] * d[~at_cut]).sum(0) if len(x) else np.zeros(3))
         mag.append((np.abs(f) * r).sum())
         edge.append((np.abs(f) * r)[at_cut].sum())
-    return np.array(out), np.array(mag), np.array(edge)
+        grad.append(np.abs(f).sum())
+        cnt.append(len(x))
+    return np.array(out), np.array(mag), np.array(edge), np.array(grad), np.array(cnt)
+
+
+def _bound(L, mag, edge, grad, cnt):
+    """The table's entries are within 1.4e-5 of a pair's force; a sum of n terms
+    rounds like 2^-24 sqrt(n) of their magnitudes (4 of these); scaled and shifted
+    coordinates put 3 x 2^-24 L into each difference, and a pair's force F r / r_p^3
+    moves by at most 3 F / r_p^3 per length."""
+    eps = 2.0 ** -24
+    return (1.4e-5 + 4 * eps * np.sqrt(cnt)) * mag + 9 * eps * L * grad + edge
 
 
 def _points(kind, n, L, seed):
@@ -76,18 +88,15 @@ def _config(J, L, M, cut, theta, n):
                     r_cut=cut * r_s, mu=3.0, G_mass_plus=1.0)
 
 
-def _check(J, cfg, pp, pm, ap, am, multipoles, seed=0):
+def _check(J, cfg, pp, pm, ap, am, multipoles, extra=None, seed=0):
     pos = np.concatenate([pp, pm]).astype(np.float64)
     mm = cfg.mu * len(pp) / len(pm) if len(pp) and len(pm) else cfg.mu
     q = np.concatenate([np.full(len(pp), 1.0), np.full(len(pm), -float(np.float32(mm)))])
     acc = np.concatenate([ap, am]).astype(np.float64)
     t = np.random.default_rng(seed).choice(len(pos), min(len(pos), 60), replace=False)
-    f, mag, edge = _short(pos, q, t, cfg.box_L, cfg.r_s, cfg.r_cut, cfg.softening)
+    f, mag, *rest = _short(pos, q, t, cfg.box_L, cfg.r_s, cfg.r_cut, cfg.softening)
     err = np.linalg.norm(acc[t] - f, axis=1)
-    # each pair's table entry is within 1.4e-5 of its force, its sum's rounding
-    # within 1e-6 of the magnitudes, and a coordinate near L/2 carries 6e-8 of
-    # it into differences of neighbours (relative to the softening at worst)
-    bound = (2e-5 + 1e-7 * cfg.box_L / cfg.softening) * mag + edge
+    bound = _bound(cfg.box_L, mag, *rest) + (0.0 if extra is None else np.concatenate(extra)[t])
     if multipoles:   # nodes of the tree walk at this theta, against the force itself
         bound = bound + 5e-3 * np.linalg.norm(f, axis=1) + 1e-4 * np.median(mag)
     assert np.all(np.isfinite(acc)) and np.all(err <= bound + 1e-30), (err / np.maximum(bound, 1e-30)).max()
@@ -109,7 +118,9 @@ def test_short_range_force(kind, n_p, n_m, L, M, cut, theta):
 
 def test_boxes_of_every_route_in_one_pass():
     """Boxes without a cell grid (r_cut > L / 3), small and clustered ones share
-    the pass's cell and batch tables."""
+    the pass's cell and batch tables.  The mesh part, taken out as a box alone
+    computes it, leaves the pairs' force on every particle that is checked, inside
+    the clumps and outside."""
     import janus_treepm as J
     rows = [CASES[4], ("uniform", 300, 200, 8.0, 16, 2.4, 0.0), CASES[9], CASES[1], CASES[8]]
     cfgs = [_config(J, L, M, cut, th, n_p + n_m) for _, n_p, n_m, L, M, cut, th in rows]
@@ -120,17 +131,24 @@ def test_boxes_of_every_route_in_one_pass():
     B.forces(ids, J.JT_PART_SHORT)
     B.forces(ids)                      # the second pass meets the first one's tables
     full = [B.accel(i) for i in ids]
-    B.forces(ids, J.JT_PART_PM)
     B.close()
-    for c, (pp, pm), (ap, am) in zip(cfgs, pts, full):
+    for row, c, (pp, pm), acc in zip(rows, cfgs, pts, full):
         s = J.Solver(c)
         s.set_state(pp, None, pm, None)
-        rp, rm = s.accel()
+        mesh, alone = s.accel_part(J.JT_PART_PM), s.accel()
         s.close()
-        for a, r in ((ap, rp), (am, rm)):
-            if len(r):
-                rms = max(float(np.sqrt((r.astype(np.float64) ** 2).sum(1).mean())), 1e-30)
-                assert np.abs(a - r).max() <= 2e-5 * max(rms, float(np.abs(r).max()))
+        tree = row is rows[2]
+        short = [a.astype(np.float64) - m for a, m in zip(acc, mesh)]
+        # the mesh force twice (32-bit FFTs): 1e-5 of its largest value in the box
+        peak = max(float(np.abs(m).max()) for m in mesh if len(m))
+        extra = [np.full(len(a), 1e-5 * peak) for a in acc]
+        for seed in (0, 1):
+            _check(J, c, pp, pm, *short, multipoles=tree or row is rows[1], extra=extra, seed=seed)
+        for a, r in zip(acc, alone):
+            if len(r):   # every particle, against its own force or the box's median
+                size = np.linalg.norm(r.astype(np.float64), axis=1)
+                diff = np.linalg.norm(a.astype(np.float64) - r, axis=1)
+                assert np.all(diff <= 1e-4 * np.maximum(size, np.median(size))), (diff / np.maximum(size, np.median(size))).max()
 
 
 def test_first_pass_of_a_large_clustered_box_counts_its_candidates():
@@ -216,11 +234,10 @@ def test_route_of_clumps_in_a_uniform_box(n, L, M, clumps, per, theta, tree):
     inside = rng.integers(0, clumps * per // 2, 10)
     for t, multipoles in ((np.concatenate([inside, n + inside]), tree),
                           (rng.integers(n - n // 8, n, 10), False)):
-        f, mag, edge = _short(pos, q, t, L, r_s, cfg.r_cut, cfg.softening)
+        f, mag, *rest = _short(pos, q, t, L, r_s, cfg.r_cut, cfg.softening)
         err = np.linalg.norm(acc[t] - f, axis=1)
-        # the table and the sums of the cell walk (2e-5 of the magnitudes); nodes at
-        # this theta: 5e-3 of the force, 1e-4 of what the clump's pairs add up to
-        bound = 2e-5 * mag + edge + (5e-3 * np.linalg.norm(f, axis=1) + 1e-4 * mag if multipoles else 0.0)
+        # nodes at this theta: 5e-3 of the force, 1e-4 of what the clump's pairs add up to
+        bound = _bound(L, mag, *rest) + (5e-3 * np.linalg.norm(f, axis=1) + 1e-4 * mag if multipoles else 0.0)
         assert np.all(err <= bound), (multipoles, (err / bound).max(), c)
 
 
@@ -247,7 +264,7 @@ def test_a_dense_clump_in_a_uniform_box_keeps_its_digits():
     pos = np.concatenate(pts).astype(np.float64)
     q = np.concatenate([np.ones(n), -np.ones(n)])
     t = np.arange(0, k, k // 60)
-    f, mag, _ = _short(pos, q, t, L, r_s, cfg.r_cut, cfg.softening)
+    f, mag, *_ = _short(pos, q, t, L, r_s, cfg.r_cut, cfg.softening)
     err = np.linalg.norm(ap[t] - f) / np.linalg.norm(f)
     # each pair rounded once or twice (2^-24), the table without bias; 1e-5 here
     assert err < 2.0 * 2.0 ** -24 * np.linalg.norm(mag) / np.linalg.norm(f), err
