@@ -171,9 +171,10 @@ constexpr int kRoundBits = 0x4B400000;
 
 // A crowded tile's particles (a clump: many per cell), one at a time by whole
 // warps: lane (a, b, c) = (lane & 3, lane >> 2 & 3, lane >> 4) adds the
-// stencil's nodes x = a, y = b, z = c and c + 2.  A row step moves 24 banks and
-// a plane step 4 (the padded pitch), so the 32 atomics of an instruction go to
-// 32 banks, wherever the particle lies and whatever its neighbours do.  (One
+// stencil's nodes x = a, y = b, z = c and c + 2.  In a 16^3 tile a row step moves
+// 24 banks and a plane step 4 (the padded pitch), so the 32 atomics of an
+// instruction go to 32 banks, wherever the particle lies and whatever its
+// neighbours do (in an 8^3 tile, of small passes, rows b and b + 2 share banks).  (One
 // particle per lane met up to 32 lanes in one cell inside a clump.)  The
 // stencils of 8 particles are computed first, one lane per particle and axis,
 // and left in the warp's scratch as the 16 products wx wy and the z weights
