@@ -47,10 +47,10 @@ UNIT = "particle-steps/s"
 # candidates outside r_cut, are overhead and not counted as useful work.
 FLOPS_PAIR = 40.0
 FLOPS_NODE = 100.0
-# DRAM bytes of one k_walk_cell launch per particle, from ncu on the 2x112^3
-# case at the same density and cut (profiles/k_walk_cell_2x112.md: 206.6 MB
-# read + 65.5 MB written for 2,809,856 particles); it grows with N
-WALK_DRAM_BYTES_PER_PARTICLE = 96.8
+# DRAM bytes of one k_walk_cell launch (with the kick) per particle, from ncu on
+# the 2x112^3 case at the same density and cut (profiles/k_walk_cell_2x96.md:
+# 210.5 MB read + 62.8 MB written for 2,809,856 particles); it grows with N
+WALK_DRAM_BYTES_PER_PARTICLE = 97.3
 # Force errors |a - a_ref| / |a_ref| (p50, p99) of this engine on B200 at the
 # benchmark configs, recorded by tests/test_gpu_accuracy_full.py (65,536
 # seeded targets against the FP64 periodic sum, "full", and the truncated
