@@ -1332,6 +1332,9 @@ struct CellWarpSmem {
     __align__(16) float cx[64], cy[64], cz[64], cq[64];
     float4 shift[kCellRanges];    // periodic shift of a range's particles
     float4 box[2];                // the targets' box (centre, widened cut^2; half sides, position scale)
+    // split batches: lanes whose target lies in a crowded block, c over the position scale
+    unsigned crowd;
+    float rest;
     int2 range[kCellRanges];      // (first, count)
 };
 
@@ -1433,8 +1436,8 @@ __device__ __forceinline__ void ld_inside(float2& ab, const float2* __restrict__
 // The differences, y and the weights of two candidates take one packed FP32
 // instruction each; the packed unit runs at half the scalar rate, so the FMA
 // pipe's time is unchanged.  Together with the batches (above): 2x224^3
-// 12.8 -> 9.2 ms at a cut of 4.5 r_s and 21.5 -> 16.6 ms at 6 r_s, 2x96^3
-// 0.86 -> 0.62 ms, 2 x 16^3 0.126 -> 0.023 ms.
+// 12.8 -> 9.4 ms at a cut of 4.5 r_s and 21.5 -> 17.0 ms at 6 r_s, 2x96^3
+// 0.86 -> 0.63 ms, 2 x 16^3 0.126 -> 0.024 ms.
 template <bool SCR, bool CNT>
 __device__ __forceinline__ unsigned cell_chunk(const CellWarpSmem& S, int cnt, CellTarget& T,
                                                const float2* __restrict__ yt)
@@ -1556,14 +1559,20 @@ __global__ void __launch_bounds__(kWarps * 32, kCellMinBlocks) k_walk_cell(CellA
             // what positions are scaled by: c, or the power of two below it, which
             // rounds nothing (and keeps the squares of any box's lengths in range)
             const float ps = raw ? __uint_as_float(__float_as_uint(cc) & 0x7f800000u) : cc;
-            const float cps = cc / ps;   // 1, or c over that power of two
+            // 1, or c over that power of two (c's significand)
+            const float cps = raw ? __uint_as_float((__float_as_uint(cc) & 0x007fffffu) | 0x3f800000u) : 1.0f;
             // this lane's target lies in a crowded block: its sum is cut into chunks
             const bool chunked =
                 raw && (A.cb.dense[(B.cbase + (int64_t)col * nbx + cell_of(p.x, B.halfL, B.cellx_inv, nbx)) >> 3] &
                         JT_BLOCK_CROWD);
+            const unsigned crowd = __ballot_sync(0xffffffffu, chunked);
             // the filter's uniform values live in shared memory: they are read
             // once per 32 candidates and would spill the pair loop's registers
             if (lane == 0) {
+                if (SPLIT > 1) {
+                    S.crowd = crowd;
+                    S.rest = cps;
+                }
                 S.box[0] = make_float4(gcx, gcy, gcz, rc2_keep);
                 S.box[1] = make_float4(ghx, ghy, ghz, ps);
             }
@@ -1613,13 +1622,24 @@ __global__ void __launch_bounds__(kWarps * 32, kCellMinBlocks) k_walk_cell(CellA
                 if (nc >= 32) {
                     hits += cell_chunk<SCR, CNT>(S, 32, T, yt);
                     cands += 32;
-                    if (raw) {
-                        // the list runs through a clump from one side to the
-                        // other, so a sum of its tens of thousands of pairs
-                        // passes far above its end: a crowded target's chunks are
-                        // summed on their own (error in overlapping clumps 1.3e-5
-                        // -> 2.8e-6 of the force).  Where chunks end depends on the
-                        // batch.  (Selects: a branch per lane takes 2 % more in a small clustered box.)
+                    // The list runs through a clump from one side to the other, so
+                    // a sum of its tens of thousands of pairs passes far above its
+                    // end: a crowded target's chunks are summed on their own (error
+                    // in overlapping clumps 1.3e-5 -> 2.8e-6 of the force).  Where
+                    // chunks end depends on the batch.  (Selects on a flag kept in a
+                    // register in whole batches, 2x224^3 9.34 against 9.57 ms with
+                    // the flags in shared memory; the other way round in split ones,
+                    // which wait for the longest batch: 2 x 12,000 clustered
+                    // particles 160 against 169 us.)
+                    if (SPLIT > 1) {
+                        const unsigned cm = S.crowd;
+                        if (cm && ((cm >> lane) & 1u)) {
+                            near.x += T.ax;
+                            near.y += T.ay;
+                            near.z += T.az;
+                            T.ax = T.ay = T.az = 0.0f;
+                        }
+                    } else if (raw) {
                         near.x += chunked ? T.ax : 0.0f;
                         near.y += chunked ? T.ay : 0.0f;
                         near.z += chunked ? T.az : 0.0f;
@@ -1655,7 +1675,7 @@ __global__ void __launch_bounds__(kWarps * 32, kCellMinBlocks) k_walk_cell(CellA
                 hits += cell_chunk<SCR, CNT>(S, (nc + 3) & ~3, T, yt);
                 cands += nc;
             }
-            const float sc = si * c2 * cps;   // sum w d, d scaled by ps
+            const float sc = si * c2 * (SPLIT > 1 ? S.rest : cps);   // sum w d, d scaled by ps
             near = Acc3{(near.x + T.ax) * sc, (near.y + T.ay) * sc, (near.z + T.az) * sc};
         }
     }
