@@ -1436,7 +1436,7 @@ __device__ __forceinline__ void ld_inside(float2& ab, const float2* __restrict__
 // The differences, y and the weights of two candidates take one packed FP32
 // instruction each; the packed unit runs at half the scalar rate, so the FMA
 // pipe's time is unchanged.  Together with the batches (above): 2x224^3
-// 12.8 -> 9.4 ms at a cut of 4.5 r_s and 21.5 -> 17.0 ms at 6 r_s, 2x96^3
+// 12.8 -> 9.3 ms at a cut of 4.5 r_s and 21.5 -> 16.9 ms at 6 r_s, 2x96^3
 // 0.86 -> 0.63 ms, 2 x 16^3 0.126 -> 0.024 ms.
 template <bool SCR, bool CNT>
 __device__ __forceinline__ unsigned cell_chunk(const CellWarpSmem& S, int cnt, CellTarget& T,
